@@ -21,6 +21,7 @@
 #include <thrust/iterator/counting_iterator.h>
 
 #include "batch_kernels.cuh"
+#include "color_flow.cuh"
 #include "gate.cuh"
 #include "persist.cuh"
 #include "recolor.cuh"
@@ -460,7 +461,7 @@ class Engine {
   int launch_sweep(const Level &L, const Step &st, SweepArgs a, bool ordered, Probes *pr);
   int launch_apply(const ClassSched &cs, bool ordered);
   int launch_modularity(const Level &L, const int32_t *Cm, const double *ownw);
-  int color_jp(const Level &L, int *ncolors, const int32_t *key = nullptr);
+  int color_jp(const Level &L, int *ncolors);
   int run_persistent(const Level &L, const std::vector<ClassSched> &sched, SweepArgs a,
                      bool jacobi, double lower, double thresh, double *mod, int *itr);
   bool persistent() const {
@@ -867,38 +868,48 @@ int Engine::vbase(const Level &L, int ncolors, int type, long *moves) {
 }
 
 // Verify mode: Jones-Plassmann in vertex-id priority = the reference's
-// one-thread sequential first-fit.
-int Engine::color_jp(const Level &L, int *ncolors, const int32_t *key) {
-  int32_t *pending, *f0, *f1, *fcount, *status, *maxc;
-  TRY(alloc(&pending, L.nv)); TRY(alloc(&f0, L.nv)); TRY(alloc(&f1, L.nv));
-  TRY(alloc(&fcount, 3)); TRY(alloc(&status, 2)); TRY(alloc(&maxc, 1));
-  CK(cudaMemsetAsync(fcount, 0, 3 * sizeof(int32_t), s_));
-  CK(cudaMemsetAsync(status, 0, 2 * sizeof(int32_t), s_));
-  CK(cudaMemsetAsync(maxc, 0xff, sizeof(int32_t), s_));
+// one-thread sequential first-fit (color_flow.cuh).
+int Engine::color_jp(const Level &L, int *ncolors) {
+  ColorFlow f{};
+  f.nv = L.nv;
+  f.ptr = L.ptr;
+  f.tail = L.tail;
   // fast mode hashes the priorities (independent sets of random order);
   // GRAPPOLO_B200_COLORING=id keeps the vertex-id order of verify mode
   const char *cm = getenv("GRAPPOLO_B200_COLORING");
-  const int hashed = (mode_ != GLV_MODE_VERIFY && !(cm && !strcmp(cm, "id"))) ? 1 : 0;
-  const uint32_t seed = 0x5bd1e995u;
-  LAUNCH(k_color_init, grid_for(L.nv, 256, nsm_ * 16), 256, 0, s_, L.nv, L.ptr, L.tail, hashed,
-         seed, pending, color_, f0, fcount, key);
-  int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_color_rounds, 256, 0));
-  int grid = std::max(1, per_sm) * nsm_;
-  int64_t nv = L.nv;
-  const int64_t *ptr = L.ptr;
-  const int32_t *tail = L.tail;
-  int32_t *color = color_;
-  void *args[] = {&nv, (void *)&ptr, (void *)&tail, (void *)&hashed, (void *)&seed, &pending,
-                  &color, &f0, &f1, &fcount, &status, (void *)&key};
-  CK(cudaLaunchCooperativeKernel((void *)k_color_rounds, grid, 256, args, 0, s_));
-  ++launches_;
+  f.hashed = (mode_ != GLV_MODE_VERIFY && !(cm && !strcmp(cm, "id"))) ? 1 : 0;
+  f.seed = 0x5bd1e995u;
+  f.color = color_;
+  const int64_t next = L.nnz / 32 + L.nv + 1;
+  f.qcap = (unsigned long long)(L.nv + L.nnz / kFlowChunk + 1);
+  int32_t *maxc;
+  TRY(alloc(&f.word, L.nv)); TRY(alloc(&f.start, L.nv)); TRY(alloc(&f.ext, next));
+  TRY(alloc(&f.queue, f.qcap)); TRY(alloc(&f.ctr, 3)); TRY(alloc(&f.status, 2));
+  TRY(alloc(&maxc, 1));
+  CK(cudaMemsetAsync(f.word, 0, L.nv * sizeof(unsigned long long), s_));
+  CK(cudaMemsetAsync(f.start, 0x7f, L.nv * sizeof(int32_t), s_));
+  CK(cudaMemsetAsync(f.ext, 0, next * sizeof(uint32_t), s_));
+  CK(cudaMemsetAsync(f.queue, 0xff, f.qcap * sizeof(unsigned long long), s_));
+  CK(cudaMemsetAsync(f.ctr, 0, 3 * sizeof(unsigned long long), s_));
+  CK(cudaMemsetAsync(f.status, 0, 2 * sizeof(int32_t), s_));
+  CK(cudaMemsetAsync(maxc, 0xff, sizeof(int32_t), s_));
+  if (L.nnz > 0) {
+    TRY(merge_splits(L));
+    LAUNCH(k_flow_counts, (int)std::max<int64_t>(1, std::min<int64_t>(merge_tiles(L.nv, L.nnz),
+                                                                      nsm_ * 4)),
+           kFlowThreads, sizeof(FlowTileSmem), s_, f, L.nnz, split_row_);
+  }
+  LAUNCH(k_flow_seed, grid_for(L.nv, 256, nsm_ * 8), 256, 0, s_, f);
+  if (L.nnz > 0)
+    LAUNCH(k_color_flow, grid_for(L.nv, 32, nsm_ * 4), kFlowThreads, 0, s_, f);
   LAUNCH(k_max_color, grid_for(L.nv, 256, nsm_ * 8), 256, 0, s_, L.nv, color_, maxc);
   int32_t h[2], hm;
-  CK(cudaMemcpyAsync(h, status, sizeof(h), cudaMemcpyDeviceToHost, s_));
+  CK(cudaMemcpyAsync(h, f.status, sizeof(h), cudaMemcpyDeviceToHost, s_));
   CK(cudaMemcpyAsync(&hm, maxc, sizeof(hm), cudaMemcpyDeviceToHost, s_));
   CK(cudaStreamSynchronize(s_));
-  dfree(pending); dfree(f0); dfree(f1); dfree(fcount); dfree(status); dfree(maxc);
+  dfree(f.word); dfree(f.start); dfree(f.ext); dfree(f.queue); dfree(f.ctr); dfree(f.status);
+  dfree(maxc);
+  if (h[1]) return fail(GLV_ERR_CUDA, "colouring stopped making progress");
   if (h[0]) return fail(GLV_ERR_COLORS, "colouring needs more than 4096 colours");
   *ncolors = hm + 1;
   return GLV_OK;
@@ -3334,6 +3345,7 @@ static int set_kernel_attributes() {
       {(const void *)k_chunk_records, (int)sizeof(PermTileSmem)},
       {(const void *)k_hc_tiles, (int)sizeof(HashTileSmem)},
       {(const void *)k_row_sums_tiles, (int)sizeof(RowSumSmem)},
+      {(const void *)k_flow_counts, (int)sizeof(FlowTileSmem)},
   };
   for (const auto &k : want) {
     const cudaError_t e =

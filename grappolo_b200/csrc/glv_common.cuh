@@ -87,6 +87,13 @@ __host__ __device__ inline uint32_t mix32(uint32_t x) {
   return x;
 }
 
+// Colouring priorities: u colours before v (lower id, or lower hashed id).
+__device__ __forceinline__ bool prio_before(int32_t u, int32_t v, int hashed, uint32_t seed) {
+  if (!hashed) return u < v;
+  const uint32_t hu = mix32((uint32_t)u ^ seed), hv = mix32((uint32_t)v ^ seed);
+  return (hu < hv) || (hu == hv && u < v);
+}
+
 // FP64 gain exactly as Utility/utilityClusteringFunctions.cpp:243 evaluates
 // it, 2*(eiy - eix) - 2*degree*(ay - ax)*constant, left to right, every
 // operation rounded on its own (no FMA contraction).

@@ -478,100 +478,6 @@ __global__ void __launch_bounds__(256) k_modularity_final(int nparts, const doub
 }
 
 // ---------------------------------------------------------------------------
-// Distance-1 colouring by priority order (Jones-Plassmann).  A vertex takes
-// the smallest colour not used by its higher-priority neighbours once they are
-// all coloured.  With priority "lower id first" this is exactly the
-// sequential first-fit pass of Coloring/coloringDistanceOne.cpp:137-150 at one
-// thread; with hashed priorities it is the parallel independent-set form.
-// With `key` given, priority is (key, id): the iterated-greedy recolouring
-// orders vertices by their previous colour class.
-__device__ __forceinline__ bool prio_before(int32_t u, int32_t v, int hashed, uint32_t seed,
-                                            const int32_t *key = nullptr) {
-  if (key) {
-    const int32_t ku = key[u], kv = key[v];
-    return (ku < kv) || (ku == kv && u < v);
-  }
-  if (!hashed) return u < v;
-  const uint32_t hu = mix32((uint32_t)u ^ seed), hv = mix32((uint32_t)v ^ seed);
-  return (hu < hv) || (hu == hv && u < v);
-}
-
-__global__ void k_color_init(int64_t nv, const int64_t *ptr, const int32_t *tail, int hashed,
-                             uint32_t seed, int32_t *pending, int32_t *color, int32_t *frontier,
-                             int32_t *fcount, const int32_t *key) {
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv;
-       v += (int64_t)gridDim.x * blockDim.x) {
-    int32_t cnt = 0;
-    for (int64_t j = ptr[v]; j < ptr[v + 1]; ++j) {
-      const int32_t u = tail[j];
-      if (u != (int32_t)v && prio_before(u, (int32_t)v, hashed, seed, key)) ++cnt;
-    }
-    pending[v] = cnt;
-    color[v] = -1;
-    if (cnt == 0) frontier[atomicAdd(fcount, 1)] = (int32_t)v;
-  }
-}
-
-// Persistent cooperative kernel: one grid-wide barrier per round.  fcount has
-// three counters used round-robin (read / push / reset).  Each round colours
-// at least one vertex, so the loop ends after at most nv rounds.
-__global__ void __launch_bounds__(256) k_color_rounds(int64_t nv, const int64_t *ptr,
-                                                      const int32_t *tail, int hashed,
-                                                      uint32_t seed, int32_t *pending,
-                                                      int32_t *color, int32_t *front0,
-                                                      int32_t *front1, int32_t *fcount,
-                                                      int32_t *status, const int32_t *key) {
-  cg::grid_group grid = cg::this_grid();
-  __shared__ uint32_t bm[8][kMaxColors / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  uint32_t *mybm = bm[warp];
-  for (int64_t round = 0; round <= nv; ++round) {
-    int32_t *cur = (round & 1) ? front1 : front0;
-    int32_t *nxt = (round & 1) ? front0 : front1;
-    const int32_t n = *((volatile int32_t *)&fcount[round % 3]);
-    if (n == 0) break;
-    if (blockIdx.x == 0 && threadIdx.x == 0) fcount[(round + 2) % 3] = 0;
-    for (int64_t k = wid; k < n; k += nw) {
-      const int32_t v = cur[k];
-      const int64_t rb = ptr[v], re = ptr[v + 1];
-      const int64_t deg = re - rb;
-      const int words = (int)((deg + 32) / 32 < kMaxColors / 32 ? (deg + 32) / 32 : kMaxColors / 32);
-      for (int q = lane; q < words; q += 32) mybm[q] = 0u;
-      __syncwarp();
-      for (int64_t j = rb + lane; j < re; j += 32) {
-        const int32_t u = tail[j];
-        if (u != v && prio_before(u, v, hashed, seed, key)) {
-          const int32_t cu = color[u];
-          if (cu >= 0 && cu < words * 32) atomicOr(&mybm[cu >> 5], 1u << (cu & 31));
-        }
-      }
-      __syncwarp();
-      int first = INT32_MAX;
-      for (int q = lane; q < words; q += 32) {
-        const uint32_t free_bits = ~mybm[q];
-        if (free_bits) { first = q * 32 + __ffs(free_bits) - 1; break; }
-      }
-      first = __reduce_min_sync(FULL, first);
-      if (first == INT32_MAX) first = words * 32;  // all marked: next colour
-      if (first >= kMaxColors) {
-        if (lane == 0) atomicExch(status, 1);
-        first = kMaxColors - 1;
-      }
-      if (lane == 0) color[v] = first;
-      __syncwarp();
-      for (int64_t j = rb + lane; j < re; j += 32) {
-        const int32_t u = tail[j];
-        if (u != v && prio_before(v, u, hashed, seed, key)) {
-          if (atomicSub(&pending[u], 1) == 1) nxt[atomicAdd(&fcount[(round + 1) % 3], 1)] = u;
-        }
-      }
-    }
-    grid.sync();
-  }
-}
-
 // Coloring/coloringMultiHashMaxMin.cpp:124-160: one (iteration, hash) pass of
 // the incomplete max/min colouring.  An uncoloured vertex (colour maxColor)
 // takes `cur` when its random value beats every neighbour not coloured in an
