@@ -209,8 +209,8 @@ struct Level {
 // One (class, sublevel) step: member positions of each degree bin.
 struct Step {
   int64_t seg[NBINS + 1];
-  int64_t hub_chunk[2] = {0, 0};  // k_hub_accum work items
-  int64_t hub_segs[2] = {0, 0};   // k_hub_scan work items
+  int64_t hub_chunk[2] = {0, 0};  // hub chunks
+  int64_t hub_segs[2] = {0, 0};   // hub partitions
 };
 
 struct ClassSched {
@@ -455,7 +455,7 @@ class Engine {
   int merge_splits(const Level &L);
   int build_schedule(const Level &L, const int32_t *color, int ncolors, const int32_t *sub,
                      int nsub, std::vector<ClassSched> *sched, bool hubs = true);
-  int hub_offsets(const Level &L, std::vector<ClassSched> &sched);
+  int hub_offsets(const Level &L, std::vector<ClassSched> &sched, bool tables);
   int group_classes(const Level &L, int ncolors, std::vector<ClassSched> *sched);
   int sublevels(const Level &L, int ncolors, int32_t **d_sub, int *nsub);
   int launch_sweep(const Level &L, const Step &st, SweepArgs a, bool ordered, Probes *pr);
@@ -498,11 +498,15 @@ class Engine {
   int32_t *hub_keys_ = nullptr;
   double *hub_vals_ = nullptr;
   size_t hub_cap_ = 0;
-  // parallel hub path (per member slot arrays, work lists, filled-slot lists)
-  int64_t *hub_occ_off_ = nullptr, *hub_seg_beg_ = nullptr, *hub_seg_end_ = nullptr;
-  int32_t *hub_cnt_ = nullptr, *hub_left_ = nullptr, *hub_big_ = nullptr, *step_big_ = nullptr;
-  int32_t *hub_segs_left_ = nullptr, *hub_err_ = nullptr;
-  uint32_t *hub_state_ = nullptr;
+  // parallel hub path (hub.cuh)
+  HubInfo *hubs_ = nullptr;
+  HubChunk *hub_chunks_ = nullptr;
+  HubState *hub_state_ = nullptr;
+  int32_t *part_hub_ = nullptr, *part_c_ = nullptr, *hub_out_c_ = nullptr, *hub_err_ = nullptr;
+  double *part_g_ = nullptr, *hub_out_w_ = nullptr;
+  uint16_t *part_off_ = nullptr;
+  int64_t nhubs_ = 0;  // hubs of the current schedule with chunks
+  size_t hubs_cap_ = 0, chunk_cap_ = 0, part_cap_ = 0, hub_out_cap_ = 0, part_off_cap_ = 0;
   uint32_t epoch_ = 0;  // persistent launches of this engine (hub states compare against it)
   int hub_chunk_ = kHubChunk;  // CSR entries per hub chunk (the autotuner may lower it)
   // trial launches of the autotuner: stop after this many iterations (0 = the
@@ -515,13 +519,6 @@ class Engine {
   int autotune(const Level &L, int ncolors, std::vector<ClassSched> *sched,
                const std::function<int(std::vector<ClassSched> *)> &make_sched, SweepArgs a,
                double lower, double thresh);
-  double *hub_self_ = nullptr, *hub_ownw_ = nullptr;
-  int32_t *hub_occ_ = nullptr;
-  size_t hub_occ_cap_ = 0;
-  int32_t *chunk_pos_ = nullptr, *seg_pos_ = nullptr, *part_c_ = nullptr;
-  int64_t *chunk_beg_ = nullptr, *chunk_end_ = nullptr, *seg_beg_ = nullptr, *seg_end_ = nullptr;
-  double *part_g_ = nullptr;
-  size_t chunk_cap_ = 0, seg_cap_ = 0;
   // Hub rows of the persistent kernel on thread-block clusters of cluster_
   // blocks (0: all hubs as chunks over global tables).  A hub whose table
   // needs at most cluster_parts_ cluster-sized partitions is a cluster row
@@ -531,26 +528,27 @@ class Engine {
   int cluster_ = 0;
   int cluster_parts_ = kClusterMaxParts;
   bool sweep_rows_ = false;
-  int32_t *ct_pos_ = nullptr, *ct_part_ = nullptr, *ct_nparts_ = nullptr, *ct_c_ = nullptr;
+  int32_t *ct_pos_ = nullptr, *ct_part_ = nullptr, *ct_nparts_ = nullptr, *ct_c_ = nullptr,
+          *ct_left_ = nullptr;
   double *ct_g_ = nullptr;
   size_t ct_cap_ = 0;
   std::vector<int32_t> hub_pos_h_;
   std::vector<int64_t> hub_deg_h_;
   int cluster_grid(int cl);  // blocks of a cooperative launch with cl-block clusters
   int cluster_grid_[kClusterMax + 1] = {};
-  bool hub_tables_clean_ = false;
   // The current colour phase runs some colour classes together in one step
   // (group_classes), so a step's members are not an independent set.
   bool relaxed_ = false;
+  // group_classes' lower row limit: 1 taken, 0 not, -1 decided by the next phase
+  int group_lower_ = 0;
+  int group_max_ = 4095;  // rows longer than this count as long there
   // Classes at and above this colour of colour_ are batches of the core (not
   // independent sets); INT32_MAX = every class is an independent set.
   int core_color_ = INT32_MAX;
   HubWork hub_work() const {
-    return HubWork{hub_keys_, hub_vals_, hub_off_, hub_occ_, hub_occ_off_, hub_cnt_, hub_self_,
-                   hub_ownw_, chunk_pos_, chunk_beg_, chunk_end_, seg_pos_, seg_beg_, seg_end_,
-                   part_g_, part_c_, hub_seg_beg_, hub_seg_end_, hub_left_, hub_big_, step_big_,
-                   hub_segs_left_, hub_state_, 0u, hub_err_, hub_chunk_, ct_pos_, ct_part_,
-                   ct_nparts_, ct_g_, ct_c_};
+    return HubWork{hubs_, hub_chunks_, part_hub_, hub_state_, hub_out_c_, hub_out_w_, part_off_,
+                   part_g_, part_c_, 0u, hub_err_, ct_pos_, ct_part_, ct_nparts_, ct_g_, ct_c_,
+                   ct_left_};
   }
   int hist_cap_ = 0;
   // ordered-delta buffers
@@ -571,6 +569,7 @@ class Engine {
   int64_t crec_cap_ = 0;
 };
 
+constexpr int kGroupLower = 2047;    // group_classes' lower row limit
 constexpr int kConstParts = 1024;  // blocks of the constant's reduction
 
 static int grid_for(int64_t n, int block, int cap) {
@@ -585,13 +584,9 @@ void Engine::release() {
                     &vals_, &move_old_, &move_new_, &hist_, &hub_keys_};
   for (auto p : ip) dfree(*p);
   dfree(hub_off_);
-  dfree(hub_occ_off_); dfree(hub_seg_beg_); dfree(hub_seg_end_); dfree(hub_cnt_);
-  dfree(hub_self_); dfree(hub_ownw_); dfree(hub_occ_); dfree(hub_left_); dfree(hub_big_);
-  dfree(hub_segs_left_); dfree(hub_state_); dfree(hub_err_);
-  dfree(step_big_); dfree(chunk_pos_); dfree(seg_pos_);
-  dfree(ct_pos_); dfree(ct_part_); dfree(ct_nparts_); dfree(ct_g_); dfree(ct_c_);
-  dfree(part_c_); dfree(chunk_beg_); dfree(chunk_end_); dfree(seg_beg_); dfree(seg_end_);
-  dfree(part_g_);
+  dfree(hubs_); dfree(hub_chunks_); dfree(hub_state_); dfree(part_hub_); dfree(part_c_);
+  dfree(part_g_); dfree(hub_out_c_); dfree(hub_out_w_); dfree(part_off_); dfree(hub_err_);
+  dfree(ct_pos_); dfree(ct_part_); dfree(ct_nparts_); dfree(ct_g_); dfree(ct_c_); dfree(ct_left_);
   dfree(dkeys_); dfree(dkeys2_); dfree(drecs_); dfree(drecs2_);
   dfree(ck1_); dfree(ck2_); dfree(cv1_); dfree(cv2_);
   dfree(rec_own_); dfree(rec_gain_); dfree(feat_); dfree(gate_p_); dfree(last_move_);
@@ -615,21 +610,13 @@ int Engine::init(int64_t nv0, int64_t nnz0) {
   TRY(alloc(&cSize, n)); TRY(alloc(&dSize, n));
   TRY(alloc(&C, n)); TRY(alloc(&Cpast, n)); TRY(alloc(&Ctgt, n)); TRY(alloc(&color_, n));
   TRY(alloc(&keys_, n)); TRY(alloc(&keys2_, n)); TRY(alloc(&members_, n)); TRY(alloc(&vals_, n));
-  TRY(alloc(&move_old_, n)); TRY(alloc(&move_new_, n)); TRY(alloc(&hub_off_, n));
-  TRY(alloc(&hub_occ_off_, n)); TRY(alloc(&hub_seg_beg_, n)); TRY(alloc(&hub_seg_end_, n));
-  TRY(alloc(&hub_cnt_, n)); TRY(alloc(&hub_self_, n)); TRY(alloc(&hub_ownw_, n));
-  TRY(alloc(&hub_left_, n)); TRY(alloc(&hub_big_, n));
-  TRY(alloc(&hub_segs_left_, n)); TRY(alloc(&hub_state_, n)); TRY(alloc(&hub_err_, 1));
-  CK(cudaMemsetAsync(hub_state_, 0, n * sizeof(uint32_t), s_));
+  TRY(alloc(&move_old_, n)); TRY(alloc(&move_new_, n)); TRY(alloc(&hub_err_, 1));
   CK(cudaMemsetAsync(hub_err_, 0, sizeof(int32_t), s_));
-  CK(cudaMemsetAsync(hub_cnt_, 0, n * sizeof(int32_t), s_));
-  CK(cudaMemsetAsync(hub_big_, 0, n * sizeof(int32_t), s_));
-  CK(cudaMemsetAsync(hub_self_, 0, n * sizeof(double), s_));
-  CK(cudaMemsetAsync(hub_ownw_, 0, n * sizeof(double), s_));
   if (const char *bm = getenv("GRAPPOLO_B200_BLOCK_MAX")) {
     const int v = atoi(bm);
     if (v >= lim_.warp_max && v <= 4095) lim_.block_max = v;
   }
+  group_max_ = lim_.block_max;
   // hub rows on clusters of this many blocks (1, 2, 4, 8 or 16; 0 = global
   // tables, the default); the autotuner may change it
   cluster_ = 0;
@@ -1128,19 +1115,47 @@ int Engine::build_schedule(const Level &L, const int32_t *color, int ncolors, co
     }
   }
   if (debug) fprintf(stderr, "grappolo_b200: schedule sort+hist %.4f s\n", now_s() - tsd);
-  return hubs ? hub_offsets(L, *sched) : GLV_OK;
+  return hubs ? hub_offsets(L, *sched, ordered()) : GLV_OK;
 }
 
-// Fast mode: colour classes whose members all have long rows (degree bin at
-// least GRAPPOLO_B200_MERGE_BIN, default the hub bin) run in steps of up to
+// Fast mode: colour classes whose members all have long rows (longer than
+// group_max_ entries, by default the block bin's limit, or of a degree bin at
+// least GRAPPOLO_B200_MERGE_BIN) run in steps of up to
 // GRAPPOLO_B200_MERGE_CLASSES classes (default 16; 0 or 1 = every class its
 // own step).  Skewed graphs colour their dense core of high-degree vertices
 // with hundreds of classes of a few vertices each, and every class is a
 // grid-wide step; a vertex of such a class has almost all of its weight on
 // vertices outside the core, so deciding a few core classes against one
 // snapshot changes little of what each decision sees.  A group takes the
-// place of its first class; the other classes keep their order.  Returns the
-// schedule rebuilt over the groups (relaxed_ set) or leaves it unchanged.
+// place of its first class; the other classes keep their order.
+// Fills map (colour -> step) for rows longer than `longer` from the schedule
+// `sched` built with that bin limit; returns the classes merged away.
+static int group_map(const std::vector<ClassSched> &sched, int ncolors, int gmax, int min_bin,
+                     std::vector<int32_t> *map, int *ngroups) {
+  map->assign(ncolors, 0);
+  int open = -1, in_open = 0, merged = 0, n = 0;
+  for (const ClassSched &cs : sched) {
+    bool long_rows = cs.steps.size() == 1;
+    for (const Step &st : cs.steps) long_rows = long_rows && st.seg[min_bin] == st.seg[0];
+    if (!long_rows) {
+      (*map)[cs.color] = n++;
+      continue;
+    }
+    if (open < 0 || in_open >= gmax) {
+      open = n++;
+      in_open = 0;
+    } else {
+      ++merged;
+    }
+    (*map)[cs.color] = open;
+    ++in_open;
+  }
+  *ngroups = n;
+  return merged;
+}
+
+// Returns the schedule rebuilt over the groups (relaxed_ set) or leaves it
+// unchanged.
 int Engine::group_classes(const Level &L, int ncolors, std::vector<ClassSched> *sched) {
   relaxed_ = false;
   if (mode_ == GLV_MODE_VERIFY || bt_ || sched->size() < 2) return GLV_OK;
@@ -1148,24 +1163,42 @@ int Engine::group_classes(const Level &L, int ncolors, std::vector<ClassSched> *
   if (const char *e = getenv("GRAPPOLO_B200_MERGE_CLASSES")) gmax = atoi(e);
   if (const char *e = getenv("GRAPPOLO_B200_MERGE_BIN")) min_bin = atoi(e);
   if (gmax <= 1 || min_bin < 0 || min_bin >= NBINS) return GLV_OK;
-  std::vector<int32_t> map(ncolors, 0);
-  int ngroups = 0, open = -1, in_open = 0, merged = 0;
-  for (const ClassSched &cs : *sched) {
-    bool long_rows = cs.steps.size() == 1;
-    for (const Step &st : cs.steps) long_rows = long_rows && st.seg[min_bin] == st.seg[0];
-    if (!long_rows) {
-      map[cs.color] = ngroups++;
-      continue;
+  std::vector<int32_t> map, map2;
+  int ngroups = 0, ng2 = 0, merged = 0, merged2 = 0;
+  bool rebuilt = false;  // the schedule's device arrays follow another limit
+  auto map_at = [&](int limit, std::vector<int32_t> *m, int *ng, int *mg) -> int {
+    if (min_bin != BIN_HUB || limit == lim_.block_max) {
+      *mg = group_map(*sched, ncolors, gmax, min_bin, m, ng);
+      return GLV_OK;
     }
-    if (open < 0 || in_open >= gmax) {
-      open = ngroups++;
-      in_open = 0;
-    } else {
-      ++merged;
+    std::vector<ClassSched> at;
+    const int block_max = lim_.block_max;
+    lim_.block_max = limit;
+    const int rc = build_schedule(L, color_, ncolors, nullptr, 1, &at, false);
+    lim_.block_max = block_max;
+    rebuilt = true;
+    *mg = group_map(at, ncolors, gmax, min_bin, m, ng);
+    return rc;
+  };
+  // On large levels a lower limit (kGroupLower) is taken when it leaves at
+  // most 7/8 of the steps: a step costs its barriers and its longest row's
+  // chain whatever it holds (R-MAT 20, edge factor 16: 199 steps and 7.2 ms a
+  // sweep with classes of rows over 4095 merged, 137 steps and 5.7 ms over
+  // 2047), but it also decides more vertices against one snapshot, so a few
+  // steps are not worth it.  The workers' own limit (lim_) plays no part: it
+  // changes no decision.
+  if (group_max_ <= kGroupLower || min_bin != BIN_HUB) group_lower_ = 0;
+  if (group_lower_ != 1) TRY(map_at(group_max_, &map, &ngroups, &merged));
+  if (group_lower_ != 0) {
+    TRY(map_at(kGroupLower, &map2, &ng2, &merged2));
+    if (group_lower_ < 0) group_lower_ = 8 * ng2 <= 7 * ngroups ? 1 : 0;
+    if (group_lower_ == 1) {
+      map.swap(map2);
+      ngroups = ng2;
+      merged = merged2;
     }
-    map[cs.color] = open;
-    ++in_open;
   }
+  if (merged == 0 && rebuilt) return build_schedule(L, color_, ncolors, nullptr, 1, sched);
   if (merged == 0) return GLV_OK;
   // colours with no member keep a slot that no vertex uses
   int32_t *d_map, *key;
@@ -1206,18 +1239,6 @@ __global__ void k_scatter_i64(int64_t n, const int32_t *pos, const int64_t *val,
     out[pos[k]] = val[k];
 }
 
-__global__ void k_hub_chunk_counts(int64_t n, const int32_t *pos, const int32_t *members,
-                                   const int64_t *ptr, const int64_t *seg_beg,
-                                   const int64_t *seg_end, int chunk, int32_t *left,
-                                   int32_t *segs_left) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t v = members[pos[k]];
-    left[pos[k]] = (int32_t)((ptr[v + 1] - ptr[v] + chunk - 1) / chunk);
-    segs_left[pos[k]] = (int32_t)(seg_end[pos[k]] - seg_beg[pos[k]]);
-  }
-}
-
 __global__ void k_row_bounds_at(int64_t n, const int32_t *pos, const int32_t *members,
                                 const int64_t *ptr, int64_t *out) {
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n;
@@ -1235,20 +1256,16 @@ static int upload(cudaStream_t s, T *dst, const std::vector<T> &src) {
   return GLV_OK;
 }
 
-// Hub tables and work lists.  Ordered accumulation (verify mode, non-integral
-// weights) walks each hub with one warp and reuses one table region per step;
-// the parallel path gives every hub of the schedule a private table, cut its
-// row into kHubChunk-entry chunks and its filled-slot list into kHubSeg
-// segments.
-constexpr size_t kHubStepSlots = size_t(1) << 28;  // hub table slots of one step (3 GB)
+// Hub tables and work lists.  With `tables` (ordered accumulation: one warp
+// walks each hub) every hub gets a table region, reused from step to step;
+// otherwise every hub's row is cut into chunks and partitions (hub.cuh).
+constexpr size_t kHubStepSlots = size_t(1) << 28;  // hub table slots or pairs of one step (3 GB)
 
-int Engine::hub_offsets(const Level &L, std::vector<ClassSched> &sched) {
-  const bool parallel = !ordered();
-  std::vector<int64_t> tab_off, occ_off, seg_b, seg_e;
-  std::vector<int32_t> c_pos, s_pos;
-  std::vector<int64_t> c_beg, c_end, s_beg, s_end;
-  std::vector<int64_t> hub_pos_all;
-  size_t need_tab = 0;
+int Engine::hub_offsets(const Level &L, std::vector<ClassSched> &sched, bool tables) {
+  std::vector<int64_t> tab_off;
+  std::vector<HubInfo> hubs;
+  std::vector<HubChunk> chunks;
+  std::vector<int32_t> part_hub;
   // row bounds of every hub of the schedule, in one gather
   std::vector<int32_t> hpos;
   for (auto &cs : sched)
@@ -1257,8 +1274,10 @@ int Engine::hub_offsets(const Level &L, std::vector<ClassSched> &sched) {
   std::vector<int64_t> hb_all(2 * hpos.size());
   hub_pos_h_.clear();
   hub_deg_h_.clear();
-  const bool cl_rows = parallel && sweep_rows_ && cluster_ > 0;
-  if (!hpos.empty()) {
+  nhubs_ = 0;
+  if (hpos.empty()) return GLV_OK;
+  const bool cl_rows = !tables && sweep_rows_ && cluster_ > 0;
+  {
     int32_t *d_pos;
     int64_t *bounds;
     TRY(alloc(&d_pos, hpos.size()));
@@ -1272,11 +1291,11 @@ int Engine::hub_offsets(const Level &L, std::vector<ClassSched> &sched) {
     dfree(d_pos);
     dfree(bounds);
   }
-  // A step whose hubs' tables would pass kHubStepSlots is cut into several
-  // steps of the same class (its other bins stay in the first): members of a
-  // class are independent and its deltas are applied after its last step, so
-  // the decisions do not change.
-  if (!hpos.empty()) {
+  // A step whose hubs' tables or pairs would pass kHubStepSlots is cut into
+  // several steps of the same class (its other bins stay in the first):
+  // members of a class are independent and its deltas are applied after its
+  // last step, so the decisions do not change.
+  {
     size_t hc = 0;
     for (auto &cs : sched) {
       std::vector<Step> out;
@@ -1287,8 +1306,8 @@ int Engine::hub_offsets(const Level &L, std::vector<ClassSched> &sched) {
         Step cur = st;
         for (int64_t k = b; k < e; ++k) {
           const int64_t deg = hb_all[2 * (hc + (k - b)) + 1] - hb_all[2 * (hc + (k - b))];
-          const size_t cap = table_cap(deg);
-          if (acc > 0 && acc + cap > kHubStepSlots) {
+          const size_t need = tables ? (size_t)table_cap(deg) : (size_t)deg;
+          if (acc > 0 && acc + need > kHubStepSlots) {
             cur.seg[BIN_HUB] = cut;
             for (int q = BIN_HUB + 1; q <= NBINS; ++q) cur.seg[q] = k;
             out.push_back(cur);
@@ -1299,7 +1318,7 @@ int Engine::hub_offsets(const Level &L, std::vector<ClassSched> &sched) {
             cut = k;
             acc = 0;
           }
-          acc += cap;
+          acc += need;
         }
         hc += (size_t)(e - b);
         out.push_back(cur);
@@ -1307,116 +1326,115 @@ int Engine::hub_offsets(const Level &L, std::vector<ClassSched> &sched) {
       cs.steps = out;
     }
   }
-  size_t hcur = 0;
-  size_t need_occ = 0;
+  size_t hcur = 0, need_tab = 0, need_out = 0, need_off = 0;
   for (auto &cs : sched)
     for (auto &st : cs.steps) {
       const int64_t b = st.seg[BIN_HUB], e = st.seg[BIN_HUB + 1];
-      st.hub_chunk[0] = st.hub_chunk[1] = (int64_t)c_pos.size();
-      st.hub_segs[0] = st.hub_segs[1] = (int64_t)s_pos.size();
+      st.hub_chunk[0] = st.hub_chunk[1] = (int64_t)chunks.size();
+      st.hub_segs[0] = st.hub_segs[1] = (int64_t)part_hub.size();
       if (e == b) continue;
       const int64_t *hb = hb_all.data() + 2 * hcur;
       hcur += (size_t)(e - b);
-      // a step's tables and filled-slot lists are empty again when it ends
-      // (the scan clears the slots it visits, the finalisation the counters),
-      // so every step starts its regions at offset 0
-      size_t step_tab = 0, step_occ = 0;
+      // A step's tables, pairs and offsets are done with when it ends, so every
+      // step starts its regions at offset 0.
+      size_t step_tab = 0, step_out = 0, step_off = 0;
+      // Chunks of hub_chunk_ entries; fewer (down to kHubChunkMin, one entry
+      // per thread) while the step's chunks would not fill the grid: a chunk of
+      // 2048 takes four rounds of its block, and the step waits for it.
+      int64_t chunk = hub_chunk_, total = 0;
+      for (int64_t k = 0; k < e - b; ++k) total += hb[2 * k + 1] - hb[2 * k];
+      while (chunk > kHubChunkMin && total < chunk * nsm_) chunk >>= 1;
       for (int64_t k = 0; k < e - b; ++k) {
         const int64_t rb = hb[2 * k], re = hb[2 * k + 1], deg = re - rb;
         const int64_t pos = b + k;
         uint32_t np = 0, cap = 0;
         if (cl_rows) cluster_row_shape(deg, cluster_, &np, &cap);
         if (cl_rows && np <= (uint32_t)cluster_parts_) {
-          // a cluster row: no global table, chunks or segments
+          // a cluster row: no chunks or partitions
           hub_pos_h_.push_back((int32_t)pos);
           hub_deg_h_.push_back(deg);
-          tab_off.push_back(0);
-          occ_off.push_back(0);
-          seg_b.push_back((int64_t)s_pos.size());
-          seg_e.push_back((int64_t)s_pos.size());
           continue;
         }
-        tab_off.push_back((int64_t)step_tab);
-        step_tab += table_cap(deg);
-        if (!parallel) continue;
-        occ_off.push_back((int64_t)step_occ);
-        step_occ += (size_t)deg + 1;
-        for (int64_t x = rb; x < re; x += hub_chunk_) {
-          c_pos.push_back((int32_t)pos);
-          c_beg.push_back(x);
-          c_end.push_back(std::min<int64_t>(re, x + hub_chunk_));
+        if (tables) {
+          tab_off.push_back((int64_t)step_tab);
+          step_tab += table_cap(deg);
+          continue;
         }
-        seg_b.push_back((int64_t)s_pos.size());
-        for (int64_t x = 0; x < deg + 1; x += kHubSeg) {
-          s_pos.push_back((int32_t)pos);
-          s_beg.push_back(x);
-          s_end.push_back(std::min<int64_t>(deg + 1, x + kHubSeg));
+        HubInfo hi;
+        hi.pos = (int32_t)pos;
+        hi.chunk0 = (int32_t)chunks.size();
+        hi.part0 = (int32_t)part_hub.size();
+        hi.nparts = hub_parts(deg);
+        const int32_t id = (int32_t)hubs.size();
+        for (int64_t x = rb; x < re; x += chunk) {
+          const int64_t len = std::min<int64_t>(chunk, re - x);
+          chunks.push_back(HubChunk{x, (int64_t)step_out, (int64_t)step_off, (int32_t)len, id});
+          step_out += (size_t)len;
+          step_off += (size_t)hi.nparts + 1;
         }
-        seg_e.push_back((int64_t)s_pos.size());
+        hi.nchunks = (int32_t)chunks.size() - hi.chunk0;
+        part_hub.insert(part_hub.end(), (size_t)hi.nparts, id);
+        hubs.push_back(hi);
       }
       need_tab = std::max(need_tab, step_tab);
-      need_occ = std::max(need_occ, step_occ);
-      st.hub_chunk[1] = (int64_t)c_pos.size();
-      st.hub_segs[1] = (int64_t)s_pos.size();
+      need_out = std::max(need_out, step_out);
+      need_off = std::max(need_off, step_off);
+      st.hub_chunk[1] = (int64_t)chunks.size();
+      st.hub_segs[1] = (int64_t)part_hub.size();
     }
-  (void)hub_pos_all;
-  if (hpos.empty()) return GLV_OK;
-  if (need_tab > hub_cap_ || (parallel && !hub_tables_clean_)) {
+  if (tables) {
     TRY(grow_hub(need_tab));
-    if (parallel) {
-      CK(cudaMemsetAsync(hub_keys_, 0xff, hub_cap_ * sizeof(int32_t), s_));
-      CK(cudaMemsetAsync(hub_vals_, 0, hub_cap_ * sizeof(double), s_));
-      hub_tables_clean_ = true;
-    }
+    if (!hub_off_) TRY(alloc(&hub_off_, (size_t)nv0_ + 1));
+    // the hubs' table offsets, scattered to their member slots
+    int32_t *d_pos;
+    int64_t *d_vals;
+    const int64_t nh = (int64_t)hpos.size();
+    TRY(alloc(&d_pos, nh));
+    TRY(upload(s_, d_pos, hpos));
+    TRY(alloc(&d_vals, nh));
+    TRY(upload(s_, d_vals, tab_off));
+    LAUNCH(k_scatter_i64, grid_for(nh, 256, nsm_ * 4), 256, 0, s_, nh, d_pos, d_vals, hub_off_);
+    CK(cudaStreamSynchronize(s_));
+    dfree(d_pos);
+    dfree(d_vals);
+    return GLV_OK;
   }
-  // per-hub values, aligned with hpos, scattered to their member slots
-  int32_t *d_pos;
-  int64_t *d_vals;
-  const int64_t nh = (int64_t)hpos.size();
-  TRY(alloc(&d_pos, nh));
-  TRY(upload(s_, d_pos, hpos));
-  TRY(alloc(&d_vals, 4 * nh));
-  TRY(upload(s_, d_vals, tab_off));
-  LAUNCH(k_scatter_i64, grid_for(nh, 256, nsm_ * 4), 256, 0, s_, nh, d_pos, d_vals, hub_off_);
-  if (parallel) {
-    if (need_occ > hub_occ_cap_) {
-      dfree(hub_occ_);
-      hub_occ_cap_ = need_occ;
-      TRY(alloc(&hub_occ_, hub_occ_cap_));
-    }
-    if (c_pos.size() > chunk_cap_) {
-      dfree(chunk_pos_); dfree(chunk_beg_); dfree(chunk_end_);
-      chunk_cap_ = c_pos.size();
-      TRY(alloc(&chunk_pos_, chunk_cap_)); TRY(alloc(&chunk_beg_, chunk_cap_));
-      TRY(alloc(&chunk_end_, chunk_cap_));
-    }
-    if (s_pos.size() > seg_cap_) {
-      dfree(seg_pos_); dfree(seg_beg_); dfree(seg_end_); dfree(part_g_); dfree(part_c_);
-      seg_cap_ = s_pos.size();
-      TRY(alloc(&seg_pos_, seg_cap_)); TRY(alloc(&seg_beg_, seg_cap_));
-      TRY(alloc(&seg_end_, seg_cap_)); TRY(alloc(&part_g_, seg_cap_)); TRY(alloc(&part_c_, seg_cap_));
-    }
-    TRY(upload(s_, chunk_pos_, c_pos)); TRY(upload(s_, chunk_beg_, c_beg));
-    TRY(upload(s_, chunk_end_, c_end)); TRY(upload(s_, seg_pos_, s_pos));
-    TRY(upload(s_, seg_beg_, s_beg)); TRY(upload(s_, seg_end_, s_end));
-    std::vector<int64_t> packed;
-    packed.reserve(3 * nh);
-    packed.insert(packed.end(), occ_off.begin(), occ_off.end());
-    packed.insert(packed.end(), seg_b.begin(), seg_b.end());
-    packed.insert(packed.end(), seg_e.begin(), seg_e.end());
-    TRY(upload(s_, d_vals + nh, packed));
-    LAUNCH(k_scatter_i64, grid_for(nh, 256, nsm_ * 4), 256, 0, s_, nh, d_pos, d_vals + nh,
-           hub_occ_off_);
-    LAUNCH(k_scatter_i64, grid_for(nh, 256, nsm_ * 4), 256, 0, s_, nh, d_pos, d_vals + 2 * nh,
-           hub_seg_beg_);
-    LAUNCH(k_scatter_i64, grid_for(nh, 256, nsm_ * 4), 256, 0, s_, nh, d_pos, d_vals + 3 * nh,
-           hub_seg_end_);
-    LAUNCH(k_hub_chunk_counts, grid_for(nh, 256, nsm_ * 4), 256, 0, s_, nh, d_pos, members_, L.ptr,
-           hub_seg_beg_, hub_seg_end_, hub_chunk_, hub_left_, hub_segs_left_);
+  nhubs_ = (int64_t)hubs.size();
+  if (hubs.empty()) return GLV_OK;
+  if (hubs.size() > hubs_cap_) {
+    dfree(hubs_); dfree(hub_state_);
+    hubs_cap_ = hubs.size();
+    TRY(alloc(&hubs_, hubs_cap_)); TRY(alloc(&hub_state_, hubs_cap_));
   }
+  if (chunks.size() > chunk_cap_) {
+    dfree(hub_chunks_);
+    chunk_cap_ = chunks.size();
+    TRY(alloc(&hub_chunks_, chunk_cap_));
+  }
+  if (part_hub.size() > part_cap_) {
+    dfree(part_hub_); dfree(part_g_); dfree(part_c_);
+    part_cap_ = part_hub.size();
+    TRY(alloc(&part_hub_, part_cap_)); TRY(alloc(&part_g_, part_cap_));
+    TRY(alloc(&part_c_, part_cap_));
+  }
+  if (need_out > hub_out_cap_) {
+    dfree(hub_out_c_); dfree(hub_out_w_);
+    hub_out_cap_ = need_out;
+    TRY(alloc(&hub_out_c_, hub_out_cap_)); TRY(alloc(&hub_out_w_, hub_out_cap_));
+  }
+  if (need_off > part_off_cap_) {
+    dfree(part_off_);
+    part_off_cap_ = need_off;
+    TRY(alloc(&part_off_, part_off_cap_));
+  }
+  std::vector<HubState> state(hubs.size());
+  for (size_t k = 0; k < hubs.size(); ++k)
+    state[k] = HubState{0.0, 0.0, 0, hubs[k].nchunks, hubs[k].nparts, 0u};
+  TRY(upload(s_, hubs_, hubs));
+  TRY(upload(s_, hub_state_, state));
+  TRY(upload(s_, hub_chunks_, chunks));
+  TRY(upload(s_, part_hub_, part_hub));
   CK(cudaStreamSynchronize(s_));
-  dfree(d_pos);
-  dfree(d_vals);
   return GLV_OK;
 }
 
@@ -1440,9 +1458,9 @@ int Engine::recolor(const Level &L, int *ncolors, int passes) {
     for (auto &cs : sched)
       for (auto &st : cs.steps) {
         StepDesc d{};
-        for (int b = 0; b <= NBINS; ++b) d.seg[b] = st.seg[b];
-        d.hub_chunk[0] = st.hub_chunk[0];
-        d.hub_chunk[1] = st.hub_chunk[1];
+        for (int b = 0; b <= NBINS; ++b) d.seg[b] = (int32_t)st.seg[b];
+        d.hub_chunk[0] = (int32_t)st.hub_chunk[0];
+        d.hub_chunk[1] = (int32_t)st.hub_chunk[1];
         steps.push_back(d);
       }
     StepDesc *d_steps;
@@ -1452,8 +1470,13 @@ int Engine::recolor(const Level &L, int *ncolors, int passes) {
     TRY(upload(s_, d_steps, steps));
     CK(cudaMemsetAsync(d_ctr, 0, steps.size() * sizeof(int64_t), s_));
     CK(cudaMemsetAsync(newc, 0xff, L.nv * sizeof(int32_t), s_));
+    uint32_t *words = nullptr;
+    if (nhubs_ > 0) {
+      TRY(alloc(&words, (size_t)nhubs_ * kColorWords));
+      CK(cudaMemsetAsync(words, 0xff, (size_t)nhubs_ * kColorWords * sizeof(uint32_t), s_));
+    }
     RecolorArgs r{L.ptr, L.tail, members_, newc, d_steps, (int)steps.size(), d_ctr,
-                  chunk_pos_, chunk_beg_, chunk_end_, hub_off_, hub_keys_, hub_left_, hub_chunk_};
+                  hubs_, hub_chunks_, hub_state_, words};
     void *args[] = {&r};
     CK(cudaLaunchCooperativeKernel((void *)k_recolor_pass, grid, kRecolorThreads, args, 0, s_));
     ++launches_;
@@ -1465,6 +1488,7 @@ int Engine::recolor(const Level &L, int *ncolors, int passes) {
     CK(cudaStreamSynchronize(s_));
     dfree(d_steps);
     dfree(d_ctr);
+    dfree(words);
     const bool gained = hm + 1 < *ncolors;
     *ncolors = hm + 1;
     if (!gained) break;
@@ -1519,12 +1543,10 @@ int Engine::launch_sweep(const Level &L, const Step &st, SweepArgs a, bool order
           const HubWork hw = hub_work();
           const int64_t nc = st.hub_chunk[1] - st.hub_chunk[0];
           const int64_t ns = st.hub_segs[1] - st.hub_segs[0];
-          LAUNCH(k_hub_accum, (int)std::min<int64_t>(nc, nsm_ * 4), 512,
-                 kHubStageSmem, s_, a, hw, st.hub_chunk[0],
-                 st.hub_chunk[1]);
-          LAUNCH(k_hub_scan, (int)std::min<int64_t>(ns, nsm_ * 8), 256, 0, s_, a, hw,
-                 st.hub_segs[0], st.hub_segs[1]);
-          LAUNCH(k_hub_final, grid_for(n * 32, 256, nsm_ * 4), 256, 0, s_, a, hw, lo, hi);
+          LAUNCH(k_hub_tasks<false>, (int)std::min<int64_t>(nc, nsm_ * 2), kHubThreads, kHubSmem,
+                 s_, a, hw, st.hub_chunk[0], st.hub_chunk[1]);
+          LAUNCH(k_hub_tasks<true>, (int)std::min<int64_t>(ns, nsm_ * 2), kHubThreads, kHubSmem,
+                 s_, a, hw, st.hub_segs[0], st.hub_segs[1]);
         }
         break;
     }
@@ -1587,6 +1609,14 @@ static int capture(cudaStream_t s, long *launches, F body, cudaGraphExec_t *exec
   return GLV_OK;
 }
 
+// Entries from which a run's first level is tuned (INT64_MAX: never).
+static int64_t tune_min_entries() {
+  const char *on = getenv("GRAPPOLO_B200_AUTOTUNE");
+  if (on && on[0] == '0') return INT64_MAX;
+  const char *mn = getenv("GRAPPOLO_B200_AUTOTUNE_MIN");
+  return mn ? atoll(mn) : (int64_t(1) << 24);
+}
+
 int Engine::coloring_phase(const Level &L, int ncolors, bool stale, double lower, double thresh,
                            double *mod, int *itr) {
   const bool debug = getenv("GRAPPOLO_B200_DEBUG") != nullptr;
@@ -1613,6 +1643,7 @@ int Engine::coloring_phase(const Level &L, int ncolors, bool stale, double lower
     sweep_rows_ = false;
     return rc;
   };
+  if (phase_index_ == 0 && !bt_ && persistent() && L.nnz >= tune_min_entries()) group_lower_ = -1;
   TRY(make_sched(&sched));
   if (debug) { cudaStreamSynchronize(s_); fprintf(stderr, "grappolo_b200: schedule %.4f s\n", now_s() - td); }
   dfree(d_sub);
@@ -1698,8 +1729,8 @@ __global__ void k_rotate(int64_t n, int32_t *past, int32_t *curr, const int32_t 
 
 // ------------------------------------------------------------- autotuner
 // Speed-only knobs of the persistent sweep, picked per graph: the degree above
-// which a row is a hub (global table, chunks over many blocks) instead of a
-// block row (8192-slot shared table), and the entries per hub chunk.  Neither
+// which a row is a hub (chunks and partitions over many blocks) instead of a
+// block row (one block), and the most entries of a hub chunk.  Neither
 // changes a decision: every candidate folds the same per-community sums
 // (exactly, on integral weights) and takes the same arg-max.  On the first
 // colour phase of a level with at least GRAPPOLO_B200_AUTOTUNE_MIN entries
@@ -1735,10 +1766,7 @@ __global__ void k_degree_log_hist(int64_t nv, const int64_t *ptr, unsigned long 
 int Engine::autotune(const Level &L, int ncolors, std::vector<ClassSched> *sched,
                      const std::function<int(std::vector<ClassSched> *)> &make_sched,
                      SweepArgs a, double lower, double thresh) {
-  const char *on = getenv("GRAPPOLO_B200_AUTOTUNE");
-  if (on && on[0] == '0') return GLV_OK;
-  const char *mn = getenv("GRAPPOLO_B200_AUTOTUNE_MIN");
-  if (L.nnz < (mn ? atoll(mn) : (int64_t(1) << 24))) return GLV_OK;
+  if (L.nnz < tune_min_entries()) return GLV_OK;
   (void)ncolors;
   // signature
   unsigned long long *d_hist;
@@ -1790,17 +1818,13 @@ int Engine::autotune(const Level &L, int ncolors, std::vector<ClassSched> *sched
   // statistics the trials must not touch
   const double s_t = t_sweep, s_e = edges_swept, s_k = sweep_kernel_s, s_b = sweep_bytes;
   const long s_l = launches_, s_s = sweep_steps, s_g = gated_iterations_;
-  // Candidates: hub thresholds 4095 and 2047 with every hub on global tables
-  // in 2048-entry chunks, 1024-entry chunks, and the hub rows that fit on
-  // 2-block clusters (the larger hubs keep their chunks).
+  // Candidates: hub thresholds 4095 and 2047, and 1024-entry chunks.  (Hub
+  // rows on 2-block clusters are not tried: 17.5 ms against 11.4 ms a sweep on
+  // R-MAT 22, 11.8 against 7.2 on R-MAT 20.)
   std::vector<TuneChoice> cands;
-  const int bms[3] = {lim0.block_max, 2047, 1023};
-  for (int bi = 0; bi < 3; ++bi) {
-    if (bms[bi] > lim0.block_max || (bi > 0 && bms[bi] == lim0.block_max)) continue;
-    if (bi < 2) cands.push_back(TuneChoice{bms[bi], kHubChunk, 0, INFINITY});
-    if (bi == 0) cands.push_back(TuneChoice{bms[bi], kHubChunk / 2, 0, INFINITY});
-    if (bi == 0 && cluster_grid(2) > 0) cands.push_back(TuneChoice{bms[bi], kHubChunk, 2, INFINITY});
-  }
+  cands.push_back(TuneChoice{lim0.block_max, kHubChunk, cluster0, INFINITY});
+  cands.push_back(TuneChoice{lim0.block_max, kHubChunk / 2, cluster0, INFINITY});
+  if (lim0.block_max > 2047) cands.push_back(TuneChoice{2047, kHubChunk, cluster0, INFINITY});
   TuneChoice best{lim0.block_max, chunk0, cluster0, INFINITY};
   int rc = GLV_OK;
   for (const TuneChoice &cand : cands) {
@@ -1950,7 +1974,7 @@ int Engine::decide(const Level &L, const int32_t *verts, int64_t nverts) {
                      s_));
   CK(cudaStreamSynchronize(s_));
   std::vector<ClassSched> sched{cs};
-  TRY(hub_offsets(L, sched));
+  TRY(hub_offsets(L, sched, true));
   SweepArgs a{};
   a.ptr = L.ptr; a.tail = L.tail; a.w = L.w; a.C = C; a.target = Ctgt; a.own_w = own_w;
   a.vDeg = vDeg; a.cDeg = cDeg; a.cSize = cSize; a.members = members_;
@@ -2028,12 +2052,6 @@ void Engine::gate_release() {
   dfree(gate_p_); dfree(evald_);
 }
 
-__global__ void k_scatter_i32(int64_t n, const int32_t *pos, const int32_t *val, int32_t *out) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-       k += (int64_t)gridDim.x * blockDim.x)
-    out[pos[k]] = val[k];
-}
-
 // Blocks of the persistent sweep kernel that a cooperative launch with
 // clusters of cl blocks keeps resident at once (whole clusters only); 0 when
 // none fits.
@@ -2086,13 +2104,15 @@ int Engine::run_persistent(const Level &L, const std::vector<ClassSched> &sched,
     for (size_t k = 0; k < cs.steps.size(); ++k) {
       const Step &st = cs.steps[k];
       StepDesc d{};
-      d.cls = (int64_t)cls_b.size() - 1;
-      for (int b = 0; b <= NBINS; ++b) d.seg[b] = st.seg[b];
-      d.hub_chunk[0] = st.hub_chunk[0]; d.hub_chunk[1] = st.hub_chunk[1];
-      d.hub_segs[0] = st.hub_segs[0]; d.hub_segs[1] = st.hub_segs[1];
+      d.cls = (int32_t)cls_b.size() - 1;
+      for (int b = 0; b <= NBINS; ++b) d.seg[b] = (int32_t)st.seg[b];
+      for (int q = 0; q < 2; ++q) {
+        d.hub_chunk[q] = (int32_t)st.hub_chunk[q];
+        d.hub_segs[q] = (int32_t)st.hub_segs[q];
+      }
       const bool last = (k + 1 == cs.steps.size());
-      d.apply[0] = last ? cs.begin : 0;
-      d.apply[1] = last ? cs.end : 0;
+      d.apply[0] = last ? (int32_t)cs.begin : 0;
+      d.apply[1] = last ? (int32_t)cs.end : 0;
       steps.push_back(d);
     }
   }
@@ -2100,10 +2120,10 @@ int Engine::run_persistent(const Level &L, const std::vector<ClassSched> &sched,
   // step's hub order; their chunk and segment lists are not used.
   const int cl = (cluster_ > 0 && !hub_pos_h_.empty()) ? cluster_ : 0;
   if (cl > 0) {
-    std::vector<int32_t> t_pos, t_part, t_np, p_pos, p_np;
+    std::vector<int32_t> t_pos, t_part, t_np;
     size_t hk = 0;
     for (auto &d : steps) {
-      d.ctask[0] = d.ctask[1] = (int64_t)t_pos.size();
+      d.ctask[0] = d.ctask[1] = (int32_t)t_pos.size();
       while (hk < hub_pos_h_.size() && hub_pos_h_[hk] < d.seg[BIN_HUB]) ++hk;
       for (; hk < hub_pos_h_.size() && hub_pos_h_[hk] < d.seg[BIN_HUB + 1]; ++hk) {
         const int32_t pos = hub_pos_h_[hk];
@@ -2114,32 +2134,24 @@ int Engine::run_persistent(const Level &L, const std::vector<ClassSched> &sched,
           t_part.push_back((int32_t)q);
           t_np.push_back((int32_t)np);
         }
-        if (np > 1) { p_pos.push_back((int32_t)pos); p_np.push_back((int32_t)np); }
       }
-      d.ctask[1] = (int64_t)t_pos.size();
+      d.ctask[1] = (int32_t)t_pos.size();
     }
     if (t_pos.size() > ct_cap_) {  // task lists and the partitioned rows' partials
-      dfree(ct_pos_); dfree(ct_part_); dfree(ct_nparts_); dfree(ct_g_); dfree(ct_c_); dfree(ct_g_); dfree(ct_c_);
+      dfree(ct_pos_); dfree(ct_part_); dfree(ct_nparts_); dfree(ct_g_); dfree(ct_c_);
+      dfree(ct_left_);
       ct_cap_ = t_pos.size();
       TRY(alloc(&ct_pos_, ct_cap_)); TRY(alloc(&ct_part_, ct_cap_)); TRY(alloc(&ct_nparts_, ct_cap_));
-      TRY(alloc(&ct_g_, ct_cap_)); TRY(alloc(&ct_c_, ct_cap_));
+      TRY(alloc(&ct_g_, ct_cap_)); TRY(alloc(&ct_c_, ct_cap_)); TRY(alloc(&ct_left_, ct_cap_));
     }
     TRY(upload(s_, ct_pos_, t_pos)); TRY(upload(s_, ct_part_, t_part));
     TRY(upload(s_, ct_nparts_, t_np));
-    if (!p_pos.empty()) {  // partitions still to finish, per partitioned row
-      int32_t *d_pp;
-      TRY(alloc(&d_pp, 2 * p_pos.size()));
-      TRY(upload(s_, d_pp, p_pos));
-      CK(cudaMemcpyAsync(d_pp + p_pos.size(), p_np.data(), p_np.size() * sizeof(int32_t),
-                         cudaMemcpyHostToDevice, s_));
-      LAUNCH(k_scatter_i32, grid_for((int64_t)p_pos.size(), 256, nsm_ * 4), 256, 0, s_,
-             (int64_t)p_pos.size(), d_pp, d_pp + p_pos.size(), hub_segs_left_);
-      CK(cudaStreamSynchronize(s_));
-      dfree(d_pp);
-    }
+    // partitions still to finish, at each row's first task
+    TRY(upload(s_, ct_left_, t_np));
+    CK(cudaStreamSynchronize(s_));
   }
   StepDesc *d_steps = nullptr;
-  int64_t *d_ctr = nullptr;
+  unsigned *d_ctr = nullptr;
   TRY(alloc(&d_steps, steps.size()));
   TRY(alloc(&d_ctr, 3 * steps.size()));  // block, team and cluster queues of every step
   TRY(upload(s_, d_steps, steps));
@@ -2338,7 +2350,7 @@ int Engine::run_persistent(const Level &L, const std::vector<ClassSched> &sched,
         if (bt->h_act[g]) batch_edges += (double)bt->gnnz[g];
     }
     p.exx_mode = (carry_exx && n >= 2) ? (check_exx ? 2 : 1) : 0;
-    cudaError_t e = cudaMemsetAsync(d_ctr, 0, 3 * steps.size() * sizeof(int64_t), s_);
+    cudaError_t e = cudaMemsetAsync(d_ctr, 0, 3 * steps.size() * sizeof(unsigned), s_);
     p.h.epoch = ++epoch_;
     if (e0) cudaEventRecord(e0, s_);
     if (e == cudaSuccess && cl > 0) {
@@ -2370,7 +2382,7 @@ int Engine::run_persistent(const Level &L, const std::vector<ClassSched> &sched,
     if (h_mod_[4] != 0.0) {
       rc = fail(GLV_ERR_CUDA, h_mod_[4] == 2.0
                                   ? "sweep: a hub partition's cluster table overflowed"
-                                  : "sweep: a hub's table scan gave up waiting for its chunks");
+                                  : "sweep: a hub's partition gave up waiting for its chunks");
       break;
     }
     if (p.exx_mode == 2) {
@@ -3341,7 +3353,8 @@ static int set_kernel_attributes() {
       {(const void *)k_sweep_block, kBlockCap * (int)(sizeof(double) + sizeof(int32_t))},
       {(const void *)k_sweep_iteration<false>, (int)kPersistSmem},
       {(const void *)k_sweep_iteration<true>, (int)kPersistSmem},
-      {(const void *)k_hub_accum, kHubStageSmem},
+      {(const void *)k_hub_tasks<false>, kHubSmem},
+      {(const void *)k_hub_tasks<true>, kHubSmem},
       {(const void *)k_chunk_records, (int)sizeof(PermTileSmem)},
       {(const void *)k_hc_tiles, (int)sizeof(HashTileSmem)},
       {(const void *)k_row_sums_tiles, (int)sizeof(RowSumSmem)},

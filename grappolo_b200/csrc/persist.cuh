@@ -8,12 +8,12 @@
 // a persistent grid takes part in every class:
 //   stage 1  hub rows on thread-block clusters (one table over the shared
 //            memory of a cluster's blocks) or, without clusters, hub chunks
-//            (global tables); rows of 1024..4095 entries per
+//            and partitions (hub.cuh); rows of 1024..4095 entries per
 //            block; rows of 128..1023 entries per 128-thread team (shared
 //            tables); then warp items (rows <= 32 entries, and 33..127-entry
 //            rows with a per-warp shared table)                  -> grid barrier
-//            (a hub with more filled slots than its last chunk's block
-//            scans is decided by scan-segment tasks of the same queue)
+//            (a hub whose last chunk's block does not decide it is decided by
+//            partition tasks of the same queue)
 //   stage 2  community totals += the class's deltas             -> grid barrier
 // (stage 2 after the class's last sublevel), then the modularity pass of the
 // iteration.
@@ -22,18 +22,22 @@
 #include <cooperative_groups.h>
 
 #include "phase_kernels.cuh"
+#include "hub.cuh"
+#include "rows.cuh"
 #include "sweep.cuh"
 
 namespace glv {
 
+// 32-bit: member positions and work items stay below 2^31.
 struct StepDesc {
-  int64_t seg[NBINS + 1];  // member positions of each degree bin
-  int64_t hub_chunk[2];    // hub accumulation work items
-  int64_t hub_segs[2];     // hub scan work items
-  int64_t apply[2];        // member range whose deltas are applied after this step
-  int64_t cls;             // colour class of the step
-  int64_t ctask[2];        // hub tasks on thread-block clusters (cluster_row_tasks)
+  int32_t seg[NBINS + 1];  // member positions of each degree bin
+  int32_t hub_chunk[2];    // hub chunks
+  int32_t hub_segs[2];     // hub partitions
+  int32_t apply[2];        // member range whose deltas are applied after this step
+  int32_t cls;             // colour class of the step
+  int32_t ctask[2];        // hub tasks on thread-block clusters (cluster_row_tasks)
 };
+constexpr int kStepWords = sizeof(StepDesc) / sizeof(int32_t);
 
 struct IterArgs {
   SweepArgs a;
@@ -50,7 +54,7 @@ struct IterArgs {
   double *cDeg;
   int32_t *cSize;
   uint64_t *trace;         // optional: globaltimer at each barrier, 4 per step + 2
-  int64_t *task_ctr;       // per step: next block, team and cluster task (zero at launch)
+  unsigned *task_ctr;      // per step: next block, team and cluster task (zero at launch)
   const int32_t *class_kept;  // gated sweeps: vertices the gate kept per class (NULL = all)
   int64_t nnz;
   const int64_t *split_row;   // merge-path tile boundaries of the level
@@ -116,19 +120,26 @@ constexpr int kPersistTableCap = 8192;  // BIN_BLOCK rows: degree <= 4095
 constexpr int kPersistWarpCap = 256;    // warp-table rows: degree <= 127
 constexpr int kTeamThreads = 128;      // team of the 128..1023-entry rows
 constexpr int kTeamCap = 2048;         // its table: table_cap(1023)
-constexpr size_t kPersistSmem = (size_t)kPersistTableCap * (sizeof(double) + sizeof(int32_t));
+constexpr int kPersistFill = 4096;      // filled-slot entries of a block: BIN_BLOCK rows
+// table values, table keys, filled slots
+constexpr size_t kPersistTableBytes =
+    (size_t)kPersistTableCap * (sizeof(double) + sizeof(int32_t));
+constexpr size_t kPersistSmem = kPersistTableBytes + kPersistFill * sizeof(uint16_t);
 static_assert(kPersistThreads / kTeamThreads * kTeamCap == kPersistTableCap,
               "team tables tile the block table");
 static_assert(kTeamThreads / 32 * kPersistWarpCap <= kTeamCap,
               "warp tables tile their team's table");
 static_assert(kPersistSmem >= sizeof(MergeSmem), "merge tiles must fit");
 static_assert(kPersistTableCap >= kClusterBlockSlots, "a cluster table part must fit");
-static_assert(kHubStageCap * (sizeof(double) + sizeof(int32_t)) <=
-                  (size_t)kPersistTableCap * sizeof(double),
-              "a hub chunk's staging values and filled-slot list sit below the table keys");
-static_assert(kPersistSmem >= (size_t)(kPersistThreads / 32) * kPersistWarpCap *
-                                  (sizeof(double) + sizeof(int32_t)),
+static_assert(kPersistTableCap == kHubTableCap && kPersistFill >= kHubList &&
+                  kPersistThreads == kHubThreads,
+              "hub tasks use the block's table and list");
+static_assert(kPersistTableBytes >= (size_t)(kPersistThreads / 32) * kPersistWarpCap *
+                                        (sizeof(double) + sizeof(int32_t)),
               "warp tables must fit in the block-table region");
+static_assert(kPersistFill / (kPersistThreads / kTeamThreads) >= 1024 && 127 < 4 * 32 &&
+                  kPersistFill >= 4096,
+              "every entry of a row has a filled-slot entry");
 
 // Community totals += the deltas the sweep accumulated (see k_apply_deltas).
 __device__ __forceinline__ void apply_deltas_range(const IterArgs &p, int64_t b, int64_t e,
@@ -188,12 +199,12 @@ template <bool kClusters>
 __global__ void __launch_bounds__(kPersistThreads, 2) k_sweep_iteration(IterArgs p) {
   cg::grid_group grid = cg::this_grid();
   extern __shared__ unsigned char smem_raw[];
-  __shared__ double s_self[32], s_g[32], sh[32];
+  __shared__ double s_self[32], s_own[32], s_g[32], sh[32];
   __shared__ int32_t s_c[32];
   const int warp = threadIdx.x >> 5, nwb = blockDim.x >> 5;
-  const int64_t ngw = (int64_t)gridDim.x * nwb;
+  const int ngw = gridDim.x * nwb;
   // warps numbered across blocks first: a step with few warp items spreads over SMs
-  const int64_t gwi = (int64_t)warp * gridDim.x + blockIdx.x;
+  const int gwi = warp * gridDim.x + blockIdx.x;
   const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t ngt = (int64_t)gridDim.x * blockDim.x;
   // shared table region: one 8192-slot table (block tasks), four 2048-slot
@@ -205,20 +216,43 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_sweep_iteration(IterArgs
   int32_t *team_keys = tkeys + (size_t)team * kTeamCap;
   double *wvals = team_vals + (size_t)(tt >> 5) * kPersistWarpCap;
   int32_t *wkeys = team_keys + (size_t)(tt >> 5) * kPersistWarpCap;
+  // filled slots: the block's, a quarter of it per team, 128 of that per warp
+  uint16_t *fill = reinterpret_cast<uint16_t *>(smem_raw + kPersistTableBytes);
+  uint16_t *team_fill = fill + (size_t)team * (kPersistFill * kTeamThreads / kPersistThreads);
+  uint16_t *wfill = team_fill + (size_t)(tt >> 5) * 128;
+  // tables are empty between tasks; every task empties the slots it filled
+  for (int q = threadIdx.x; q < kPersistTableCap; q += kPersistThreads) {
+    tkeys[q] = -1;
+    tvals[q] = 0.0;
+  }
+  __syncthreads();
   GLV_TRACE(4 * p.nsteps);
   // next task of the block and team queues, by task parity: the following
   // task is fetched when a task starts and published after it ends
-  __shared__ int64_t s_task[2];
-  __shared__ int64_t s_team_task[kPersistThreads / kTeamThreads][2];
-  __shared__ int s_flag;
-  __shared__ uint32_t s_word;
+  __shared__ int s_task[2];
+  __shared__ int s_team_task[kPersistThreads / kTeamThreads][2];
+  __shared__ HubShared s_hub;
   __shared__ ClusterShared s_cluster;
   // this block's slot of the moves' e_xx changes (only this block writes it)
   if (p.a.exx_delta && threadIdx.x == 0) p.a.exx_delta[blockIdx.x] = 0.0;
+  // The step's description in shared memory, loaded a step ahead: its values
+  // cost no registers across the tasks and no L2 round trip after a barrier.
+  __shared__ StepDesc s_step[2];
+  if (threadIdx.x < kStepWords && p.nsteps > 0)
+    reinterpret_cast<int32_t *>(&s_step[0])[threadIdx.x] =
+        reinterpret_cast<const int32_t *>(&p.steps[0])[threadIdx.x];
+  __syncthreads();
   for (int s = 0; s < p.nsteps; ++s) {
-    const StepDesc &st = p.steps[s];
-    // a class the gate emptied is skipped whole (no work, no barrier)
-    if (p.class_kept && p.class_kept[st.cls] == 0) continue;
+    const StepDesc &st = s_step[s & 1];
+    // (read after this step's barriers, or after the one below for a skipped step)
+    if (threadIdx.x < kStepWords && s + 1 < p.nsteps)
+      reinterpret_cast<int32_t *>(&s_step[(s + 1) & 1])[threadIdx.x] =
+          reinterpret_cast<const int32_t *>(&p.steps[s + 1])[threadIdx.x];
+    // a class the gate emptied is skipped whole (no work, no grid barrier)
+    if (p.class_kept && p.class_kept[st.cls] == 0) {
+      __syncthreads();
+      continue;
+    }
     // Stage 1 in three parts, each from its own queue: (A) hub chunks and
     // rows of 1024..4095 entries, whole blocks with an 8192-slot table;
     // (B) rows of 128..1023 entries, 128-thread teams (four per block, each
@@ -226,84 +260,87 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_sweep_iteration(IterArgs
     // 32 entries, several per warp; rows of 33..127 entries, one per warp),
     // item t to warp t mod (warps of the grid), in the warp's slice of its
     // team's table region.
-    const int64_t n4 = st.seg[1] - st.seg[0], n8 = st.seg[2] - st.seg[1];
-    const int64_t n16 = st.seg[3] - st.seg[2], n32 = st.seg[4] - st.seg[3];
-    const int64_t nw = st.seg[5] - st.seg[4];
-    const int64_t i4 = (n4 + 7) / 8, i8 = (n8 + 3) / 4, i16 = (n16 + 1) / 2;
-    const int64_t witems = i4 + i8 + i16 + n32 + nw;
-    const int64_t t_hub = st.hub_chunk[1] - st.hub_chunk[0];
-    const int64_t t_blk = st.seg[BIN_BLOCK + 1] - st.seg[BIN_BLOCK];
-    const int64_t t_seg = st.hub_segs[1] - st.hub_segs[0];
-    const int64_t n256 = st.seg[BIN_T256 + 1] - st.seg[BIN_T256];
-    const int64_t n128 = st.seg[BIN_T128 + 1] - st.seg[BIN_T128];
-    const int64_t t_ct = kClusters ? st.ctask[1] - st.ctask[0] : 0;
+    const int t_hub = st.hub_chunk[1] - st.hub_chunk[0];
+    const int t_blk = st.seg[BIN_BLOCK + 1] - st.seg[BIN_BLOCK];
+    const int t_seg = st.hub_segs[1] - st.hub_segs[0];
+    const int t_ct = kClusters ? st.ctask[1] - st.ctask[0] : 0;
     if constexpr (kClusters) if (t_ct > 0) {
       // hub rows on clusters (launches with a cluster dimension): every block
       // of a cluster takes part in every task of its cluster
       cluster_row_tasks(p.a, p.h, st.ctask[0], t_ct, &p.task_ctr[3 * s + 2],
-                        reinterpret_cast<int32_t *>(tvals + kPersistTableCap), tvals, &s_cluster,
-                        s_g, s_c);
+                        tkeys, tvals, &s_cluster, s_g, s_c);
       GLV_QTRACE(s, 3, threadIdx.x == 0);
     }
     if (t_hub + t_blk + t_seg > 0) {
-      // hub chunks, then block rows, then hub scan segments (which wait for
-      // their hub's chunks: every chunk is handed out before any segment)
-      unsigned long long *ctr = (unsigned long long *)&p.task_ctr[3 * s];
-      if (threadIdx.x == 0) s_task[0] = (int64_t)atomicAdd(ctr, 1ull);
+      // hub chunks, then block rows, then hub partitions (which wait for
+      // their hub's chunks: every chunk is handed out before any partition)
+      unsigned *ctr = &p.task_ctr[3 * s];
+      if (threadIdx.x == 0) s_task[0] = (int)atomicAdd(ctr, 1u);
       __syncthreads();
       for (unsigned it = 0;; ++it) {
-        const int64_t t = s_task[it & 1];
-        if (t >= t_hub + t_blk + t_seg) break;
-        const int64_t nxt = (threadIdx.x == 0) ? (int64_t)atomicAdd(ctr, 1ull) : 0;
-        if (t < t_hub) {
-          hub_accum_chunk(p.a, p.h, st.hub_chunk[0] + t,
-                          reinterpret_cast<int32_t *>(tvals + kPersistTableCap), tvals, s_self,
-                          s_g, s_c, &s_flag, s);
-        } else if (t < t_hub + t_blk) {
-          team_vertex<512>(p.a, st.seg[BIN_BLOCK] + (t - t_hub),
-                           reinterpret_cast<int32_t *>(tvals + kPersistTableCap), tvals, 0, s_self,
-                           s_g, s_c);
+        int t = s_task[it & 1];
+        if (t >= st.hub_chunk[1] - st.hub_chunk[0] + st.seg[BIN_BLOCK + 1] - st.seg[BIN_BLOCK] +
+                     st.hub_segs[1] - st.hub_segs[0])
+          break;
+        const int nxt = (threadIdx.x == 0) ? (int)atomicAdd(&p.task_ctr[3 * s], 1u) : 0;
+        if (t < st.hub_chunk[1] - st.hub_chunk[0]) {
+          hub_chunk_task(p.a, p.h, st.hub_chunk[0] + t, tkeys, tvals, fill, &s_hub, s_g, s_c);
         } else {
-          hub_segment_task(p.a, p.h, st.hub_segs[0] + (t - t_hub - t_blk), s_g, s_c, &s_word);
+          t -= st.hub_chunk[1] - st.hub_chunk[0];
+          const int nblk = st.seg[BIN_BLOCK + 1] - st.seg[BIN_BLOCK];
+          if (t < nblk)
+            row_vertex<512>(p.a, st.seg[BIN_BLOCK] + t, tkeys, tvals, fill, 0, s_self, s_own, s_g,
+                            s_c);
+          else
+            hub_part_task(p.a, p.h, st.hub_segs[0] + (t - nblk), tkeys, tvals, fill, &s_hub, s_g,
+                          s_c);
         }
         if (threadIdx.x == 0) s_task[(it + 1) & 1] = nxt;
         __syncthreads();
       }
       GLV_QTRACE(s, 0, threadIdx.x == 0);
     }
-    if (n256 + n128 > 0) {
-      unsigned long long *ctr = (unsigned long long *)&p.task_ctr[3 * s + 1];
-      if (tt == 0) s_team_task[team][0] = (int64_t)atomicAdd(ctr, 1ull);
+    if (st.seg[BIN_T256 + 1] > st.seg[BIN_T128]) {
+      if (tt == 0) s_team_task[team][0] = (int)atomicAdd(&p.task_ctr[3 * s + 1], 1u);
       team_sync<128>(team);
       for (unsigned it = 0;; ++it) {
-        const int64_t t = s_team_task[team][it & 1];
-        if (t >= n256 + n128) break;
-        const int64_t nxt = (tt == 0) ? (int64_t)atomicAdd(ctr, 1ull) : 0;
-        const int64_t pos = (t < n256) ? st.seg[BIN_T256] + t : st.seg[BIN_T128] + (t - n256);
-        team_vertex<128>(p.a, pos, team_keys, team_vals, team, s_self + 4 * team,
-                         s_g + 4 * team, s_c + 4 * team);
+        const int t = s_team_task[team][it & 1];
+        // the longer rows (the T256 bin, after the T128 bin in member order) first
+        const int n256 = st.seg[BIN_T256 + 1] - st.seg[BIN_T256];
+        if (t >= st.seg[BIN_T256 + 1] - st.seg[BIN_T128]) break;
+        const int nxt = (tt == 0) ? (int)atomicAdd(&p.task_ctr[3 * s + 1], 1u) : 0;
+        const int pos = (t < n256) ? st.seg[BIN_T256] + t : st.seg[BIN_T128] + (t - n256);
+        row_vertex<128>(p.a, pos, team_keys, team_vals, team_fill, team, s_self + 4 * team,
+                        s_own + 4 * team, s_g + 4 * team, s_c + 4 * team);
         if (tt == 0) s_team_task[team][(it + 1) & 1] = nxt;
         team_sync<128>(team);
       }
       GLV_QTRACE(s, 1, tt == 0);
     }
-    for (int64_t k = gwi; k < witems; k += ngw) {
-      int64_t q = k;
-      if (q < i4) { small_item<4>(p.a, st.seg[0] + 8 * q, st.seg[1]); continue; }
-      q -= i4;
-      if (q < i8) { small_item<8>(p.a, st.seg[1] + 4 * q, st.seg[2]); continue; }
-      q -= i8;
-      if (q < i16) { small_item<16>(p.a, st.seg[2] + 2 * q, st.seg[3]); continue; }
-      q -= i16;
-      if (q < n32) { small_item<32>(p.a, st.seg[3] + q, st.seg[4]); continue; }
-      q -= n32;
-      warp_table_vertex(p.a, st.seg[4] + q, wkeys, wvals);
+    {
+      const int i4 = (st.seg[1] - st.seg[0] + 7) / 8, i8 = (st.seg[2] - st.seg[1] + 3) / 4;
+      const int i16 = (st.seg[3] - st.seg[2] + 1) / 2;
+      const int witems = i4 + i8 + i16 + st.seg[5] - st.seg[3];
+      for (int k = gwi; k < witems; k += ngw) {
+        int q = k;
+        if (q < i4) { small_item<4>(p.a, st.seg[0] + 8 * q, st.seg[1]); continue; }
+        q -= i4;
+        if (q < i8) { small_item<8>(p.a, st.seg[1] + 4 * q, st.seg[2]); continue; }
+        q -= i8;
+        if (q < i16) { small_item<16>(p.a, st.seg[2] + 2 * q, st.seg[3]); continue; }
+        q -= i16 - st.seg[3];  // its member position
+        if (q < st.seg[4]) small_item<32>(p.a, q, st.seg[4]);
+        else
+          row_vertex<32>(p.a, q, wkeys, wvals, wfill, 0, nullptr, nullptr, nullptr, nullptr);
+      }
+      GLV_QTRACE(s, 2, (threadIdx.x & 31) == 0 && gwi < witems);
     }
-    GLV_QTRACE(s, 2, (threadIdx.x & 31) == 0 && gwi < witems);
+    // read before the barrier: past it another warp may load over this step
+    const int apply_b = st.apply[0], apply_e = st.apply[1];
     grid.sync();
     GLV_TRACE(4 * s);
-    if (!p.jacobi && st.apply[1] > st.apply[0]) {
-      apply_deltas_range(p, st.apply[0], st.apply[1], gt, ngt);
+    if (!p.jacobi && apply_e > apply_b) {
+      apply_deltas_range(p, apply_b, apply_e, gt, ngt);
       grid.sync();
       GLV_TRACE(4 * s + 3);
     }

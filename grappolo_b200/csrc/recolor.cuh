@@ -23,12 +23,10 @@ struct RecolorArgs {
   const StepDesc *steps;       // one step per class
   int nsteps;
   int64_t *task_ctr;           // per step (zero at launch)
-  const int32_t *chunk_pos;    // hub rows: chunk -> member slot
-  const int64_t *chunk_beg, *chunk_end;
-  const int64_t *hub_off;      // per member slot: offset of its hub table region
-  int32_t *hub_words;          // hub table regions, used as all-ones bitmaps here
-  int32_t *chunks_left;        // per member slot: chunks not yet folded
-  int chunk;                   // CSR entries per hub chunk
+  const HubInfo *hubs;         // hub rows and their chunks
+  const HubChunk *chunks;
+  HubState *state;             // chunks_left: chunks not yet folded
+  uint32_t *hub_words;         // per hub: an all-ones bitmap of kColorWords words
 };
 
 constexpr int kRecolorThreads = 512;
@@ -115,12 +113,13 @@ __device__ __forceinline__ void recolor_block(const RecolorArgs &r, int64_t pos,
 // takes the first colour still set and restores the words to all ones.
 __device__ __forceinline__ void recolor_hub_chunk(const RecolorArgs &r, int64_t ci, uint32_t *bm,
                                                   int *s_flag) {
-  const int32_t pos = r.chunk_pos[ci];
-  const int32_t v = r.members[pos];
-  uint32_t *gw = reinterpret_cast<uint32_t *>(r.hub_words + r.hub_off[pos]);
+  const HubChunk ch = r.chunks[ci];
+  const HubInfo hb = r.hubs[ch.hub];
+  const int32_t v = r.members[hb.pos];
+  uint32_t *gw = r.hub_words + (size_t)ch.hub * kColorWords;
   for (int q = threadIdx.x; q < kColorWords; q += blockDim.x) bm[q] = 0u;
   __syncthreads();
-  for (int64_t j = r.chunk_beg[ci] + threadIdx.x; j < r.chunk_end[ci]; j += blockDim.x) {
+  for (int64_t j = ch.beg + threadIdx.x; j < ch.beg + ch.len; j += blockDim.x) {
     const int32_t u = r.tail[j];
     const int32_t cu = (u != v) ? r.newc[u] : -1;
     if (cu >= 0 && cu < kMaxColors) atomicOr(&bm[cu >> 5], 1u << (cu & 31));
@@ -130,7 +129,7 @@ __device__ __forceinline__ void recolor_hub_chunk(const RecolorArgs &r, int64_t 
     if (bm[q]) atomicAnd(&gw[q], ~bm[q]);
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_flag[0] = (atomicSub(&r.chunks_left[pos], 1) == 1) ? 1 : 0;
+  if (threadIdx.x == 0) s_flag[0] = (atomicSub(&r.state[ch.hub].chunks_left, 1) == 1) ? 1 : 0;
   __syncthreads();
   if (!s_flag[0]) return;  // block-uniform
   __threadfence();
@@ -145,7 +144,7 @@ __device__ __forceinline__ void recolor_hub_chunk(const RecolorArgs &r, int64_t 
     for (int q = lane; q < kColorWords; q += 32) gw[q] = 0xffffffffu;
     if (lane == 0) {
       r.newc[v] = (first == INT32_MAX) ? kMaxColors - 1 : first;
-      r.chunks_left[pos] = (int32_t)((r.ptr[v + 1] - r.ptr[v] + r.chunk - 1) / r.chunk);
+      r.state[ch.hub].chunks_left = hb.nchunks;
     }
   }
   __syncthreads();

@@ -224,39 +224,14 @@ __device__ __forceinline__ uint32_t table_slot(int32_t *keys, uint32_t mask, int
   }
 }
 
-// table_slot that also tells whether this call inserted the key.
-__device__ __forceinline__ uint32_t table_slot_new(int32_t *keys, uint32_t mask, int32_t key,
-                                                   bool &fresh) {
-  uint32_t s = hash_slot(key, mask);
-  fresh = false;
-  while (true) {
-    int32_t k = keys[s];
-    if (k == key) return s;
-    if (k == -1) {
-      int32_t old = atomicCAS(&keys[s], -1, key);
-      if (old == -1) { fresh = true; return s; }
-      if (old == key) return s;
-    }
-    s = (s + 1) & mask;
-  }
-}
-
-__device__ __forceinline__ uint32_t table_find(const int32_t *keys, uint32_t mask, int32_t key) {
-  uint32_t s = hash_slot(key, mask);
-  while (keys[s] != key) s = (s + 1) & mask;
-  return s;
-}
-
 // One warp accumulates row [rb, re) into the table in CSR order.  Leaders
 // fold their group's weights starting from the table value, so each
 // community's sum is the sequential CSR-order sum.  Returns the self-loop sum
 // (same value in every lane).  With `atomic_add` the group sums are added with
-// atomics instead (used when several warps share one table).  With `fill`
-// every slot this call fills first is appended to fill[] (count in *nfill).
+// atomics instead (used when several warps share one table).
 __device__ __forceinline__ double warp_accumulate(const SweepArgs &a, int32_t v, int64_t rb,
                                                   int64_t re, int64_t stride, int32_t *keys,
-                                                  double *vals, uint32_t mask, bool atomic_add,
-                                                  int32_t *fill = nullptr, int *nfill = nullptr) {
+                                                  double *vals, uint32_t mask, bool atomic_add) {
   const int lane = threadIdx.x & 31;
   double self_loop = 0.0;
   // Software pipeline, two rounds deep: while this round is folded, the next
@@ -288,13 +263,7 @@ __device__ __forceinline__ double warp_accumulate(const SweepArgs &a, int32_t v,
     uint32_t slot = 0;
     double acc = 0.0;
     if (leader) {
-      if (fill) {
-        bool fresh;
-        slot = table_slot_new(keys, mask, c, fresh);
-        if (fresh) fill[atomicAdd(nfill, 1)] = (int32_t)slot;
-      } else {
-        slot = table_slot(keys, mask, c);
-      }
+      slot = table_slot(keys, mask, c);
       if (!atomic_add) acc = vals[slot];
     }
     unsigned rem = leader ? m : 0u;
@@ -455,63 +424,6 @@ __device__ __forceinline__ void block_vertex(const SweepArgs &a, int64_t pos, in
   __syncthreads();
 }
 
-// Team of T threads (T/32 warps; T == blockDim.x or a named-barrier slice of
-// the block) handles one row with the table in `keys`/`vals`; parallel
-// accumulation only.  `red` arrays have one entry per warp of the team.
-template <int T>
-__device__ __forceinline__ void team_sync(int team) {
-  if (T == 512) __syncthreads();
-  else asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(T) : "memory");
-}
-
-template <int T>
-__device__ __forceinline__ void team_vertex(const SweepArgs &a, int64_t pos, int32_t *keys,
-                                            double *vals, int team, double *s_self, double *s_g,
-                                            int32_t *s_c) {
-  constexpr int NW = T / 32;
-  const int tt = threadIdx.x % T;
-  const int lane = tt & 31, tw = tt >> 5;
-  const int32_t v = a.members[pos];
-  if (skipped(a, v)) {  // team-uniform
-    if (tt == 0) emit_stay(a, pos, v, a.C[v]);
-    return;
-  }
-  // the row's bounds and the vertex's own values load together, and the
-  // community totals of its own community right after: they arrive while
-  // the table is cleared and the row accumulates
-  const int64_t rb = a.ptr[v], re = a.ptr[v + 1];
-  const int32_t own = a.C[v];
-  const double degree = a.vDeg[v];
-  const double cdeg_own = a.cDeg[own];
-  const int32_t own_size = (tt == 0) ? a.cSize[own] : 0;
-  const uint32_t cap = table_cap(re - rb);
-  const uint32_t mask = cap - 1;
-  for (uint32_t s = tt; s < cap; s += T) { keys[s] = -1; vals[s] = 0.0; }
-  team_sync<T>(team);
-  if (tt == 0) keys[hash_slot(own, mask)] = own;
-  team_sync<T>(team);
-  const double sl = warp_accumulate(a, v, rb + 32 * tw, re, 32 * NW, keys, vals, mask, true);
-  if (lane == 0) s_self[tw] = sl;
-  team_sync<T>(team);
-  double self_loop = 0.0;
-  for (int k = 0; k < NW; ++k) self_loop = __dadd_rn(self_loop, s_self[k]);
-  const double own_w = vals[hash_slot(own, mask)];
-  const double eix = __dsub_rn(own_w, self_loop);
-  const double ax = __dsub_rn(cdeg_own, degree);
-  double g = 0.0;
-  int32_t bc = INT32_MAX;
-  scan_table(a, keys, vals, tt, cap, T, own, eix, ax, degree, cst_of(a, v), g, bc);
-  warp_argmax(g, bc);
-  if (lane == 0) { s_g[tw] = g; s_c[tw] = bc; }
-  team_sync<T>(team);
-  if (tt == 0) {
-    for (int k = 1; k < NW; ++k)
-      if (better(s_g[k], s_c[k], g, bc)) { g = s_g[k]; bc = s_c[k]; }
-    emit_decision(a, pos, v, own, finish_choice(a, own, own_size, g, bc), degree, own_w, g);
-  }
-  team_sync<T>(team);
-}
-
 // BIN_T128/T256/BLOCK keep the table in shared memory (capacity up to 8192),
 // BIN_HUB in global scratch at hub_off.
 __global__ void __launch_bounds__(512) k_sweep_block(SweepArgs a, int64_t begin, int64_t end,
@@ -537,378 +449,51 @@ __global__ void __launch_bounds__(512) k_sweep_block(SweepArgs a, int64_t begin,
 }
 
 // ---------------------------------------------------------------------------
-// Hubs in the parallel-accumulation modes: each hub's row is cut into chunks
-// that all blocks share (hub_accum_chunk), its table is scanned in segments of
-// the slots that were filled (hub_scan_segment), and one warp per hub folds
-// the segments' partial arg-maxes (hub_final).  Every table is left empty
-// again by the scan, so tables are cleared only when allocated.
+// Hubs in the parallel-accumulation modes (hub.cuh): the hubs of a schedule,
+// numbered densely, with their chunks and partitions.
+constexpr int kHubChunk = 2048;     // most CSR entries per chunk
+constexpr int kHubChunkMin = 512;   // fewest the schedule cuts rows into
+
+struct HubInfo {
+  int32_t pos;              // member slot
+  int32_t chunk0, nchunks;  // its chunks
+  int32_t part0, nparts;    // its partitions (nparts a power of two)
+};
+struct HubChunk {
+  int64_t beg;              // CSR range [beg, beg + len)
+  int64_t out;              // its pairs in out_c / out_w
+  int64_t off;              // its nparts + 1 partition offsets in part_off
+  int32_t len, hub;
+};
+struct HubState {
+  double self_w, own_w;     // row sums: self-loops, own community
+  int32_t cnt;              // pairs written
+  int32_t chunks_left, parts_left;
+  uint32_t state;           // 4 * epoch + 1 decided, + 2 its partitions decide
+};
 struct HubWork {
-  int32_t *keys;            // tables (keys -1 = empty)
-  double *vals;
-  const int64_t *tab_off;   // per member slot: table offset
-  int32_t *occ;             // filled-slot lists
-  const int64_t *occ_off;   // per member slot: list offset
-  int32_t *cnt;             // per member slot: filled slots
-  double *self_w;           // per member slot: self-loop weight
-  double *own_w;            // per member slot: Counter[own]
-  const int32_t *chunk_pos; // chunk -> member slot
-  const int64_t *chunk_beg, *chunk_end;  // CSR range
-  const int32_t *seg_pos;   // segment -> member slot
-  const int64_t *seg_beg, *seg_end;      // range in the filled-slot list
-  double *part_g;           // per segment: best gain
-  int32_t *part_c;          //              and its community
-  const int64_t *hub_seg_beg, *hub_seg_end;  // per member slot: its segments
-  int32_t *chunks_left;     // per member slot: chunks still accumulating
-  int32_t *big;             // per member slot: 1 = decided by the segment scan
-  int32_t *step_big;        // per step: some hub of the step is big (unused by the persistent kernel)
-  // persistent kernel: segments are tasks of their step that wait for the
-  // hub's chunks; the last segment to finish decides the hub
-  int32_t *segs_left;       // per member slot: segments not yet scanned
-  uint32_t *state;          // per member slot: 4 * epoch + 1 decided, + 2 segments needed
-  uint32_t epoch;           // this launch (0: the launch-per-kernel path, big[] instead)
-  int32_t *err;             // set when a segment's wait gives up
-  int chunk;                // CSR entries per accumulation chunk (<= kHubChunk)
+  const HubInfo *hubs;
+  const HubChunk *chunks;
+  const int32_t *part_hub;  // partition task -> hub
+  HubState *state;
+  int32_t *out_c;           // pairs of the step's chunks
+  double *out_w;
+  uint16_t *part_off;
+  double *part_g;           // per partition task: best gain
+  int32_t *part_c;          //                     and its community
+  uint32_t epoch;           // this launch of the persistent kernel (0: a launch per kernel)
+  int32_t *err;             // set when a partition's wait gives up
   // persistent kernel on thread-block clusters (cluster_row_tasks): the hub
   // rows' tasks, one per (row, community partition); a partitioned row's
-  // partial bests are ct_g/ct_c[task] and segs_left[member slot] counts its
+  // partial bests are ct_g/ct_c[task], and ct_left[its first task] counts its
   // partitions not yet done
   const int32_t *ct_pos;    // task -> member slot
   const int32_t *ct_part;   // task -> partition index
   const int32_t *ct_nparts; // task -> partitions of its row (a power of two)
   double *ct_g;             // task -> best gain of its partition
   int32_t *ct_c;            //         and its community
+  int32_t *ct_left;
 };
-
-constexpr int kHubChunk = 2048;      // most CSR entries per accumulation work item
-constexpr int kHubSeg = 8192;        // filled slots per scan work item
-constexpr int kHubStageCap = 4096;   // block-local staging table of one chunk
-constexpr int kHubInlineCap = 4096;  // filled slots the last chunk's block scans itself
-constexpr int kHubBatch = 4;         // table slots a thread has in flight at once
-static_assert(kHubChunk < kHubStageCap, "a chunk's distinct keys must fit the staging table");
-// staging values, the filled-slot list and staging keys of one chunk
-constexpr int kHubStageSmem = kHubStageCap * (int)(sizeof(double) + 2 * sizeof(int32_t));
-
-// Best (gain, id) over the filled slots occ[k0..k1) of a hub table; the slots
-// are emptied for the table's next use.  kHubBatch slots per thread are
-// loaded before any is used, so the occ -> key -> cDeg chains overlap.
-__device__ __forceinline__ void hub_scan_slots(const SweepArgs &a, int32_t *keys, double *vals,
-                                               const int32_t *occ, int64_t k0, int64_t k1,
-                                               int32_t own, double eix, double ax, double degree,
-                                               double cst, double &g, int32_t &bc) {
-  for (int64_t kb = k0 + threadIdx.x; kb < k1; kb += (int64_t)kHubBatch * blockDim.x) {
-    int32_t s[kHubBatch], c[kHubBatch];
-    double val[kHubBatch], cd[kHubBatch];
-#pragma unroll
-    for (int j = 0; j < kHubBatch; ++j) {
-      const int64_t k = kb + (int64_t)j * blockDim.x;
-      s[j] = (k < k1) ? __ldcg(&occ[k]) : -1;
-    }
-#pragma unroll
-    for (int j = 0; j < kHubBatch; ++j) {
-      c[j] = (s[j] >= 0) ? __ldcg(&keys[s[j]]) : -1;
-      val[j] = (s[j] >= 0) ? __ldcg(&vals[s[j]]) : 0.0;
-    }
-#pragma unroll
-    for (int j = 0; j < kHubBatch; ++j) cd[j] = (c[j] >= 0 && c[j] != own) ? a.cDeg[c[j]] : 0.0;
-#pragma unroll
-    for (int j = 0; j < kHubBatch; ++j) {
-      if (s[j] < 0) continue;
-      if (c[j] != own) {
-        const double gain = louvain_gain(val[j], eix, degree, cd[j], ax, cst);
-        if (gain > 0.0 && better(gain, c[j], g, bc)) { g = gain; bc = c[j]; }
-      }
-      keys[s[j]] = -1;
-      vals[s[j]] = 0.0;
-    }
-  }
-}
-
-// All threads of the block call.  The chunk is first folded into a
-// block-local shared table (`skeys`/`svals`, kHubStageCap slots; at most
-// kHubChunk distinct keys), then each distinct community is added to the
-// hub's global table once — a hub's neighbours concentrate on a few
-// communities, and per-warp global atomics on those slots would serialise.
-__device__ __forceinline__ void hub_accum_chunk(const SweepArgs &a, const HubWork &h, int64_t ci,
-                                                int32_t *skeys, double *svals, double *s_self,
-                                                double *s_g, int32_t *s_c, int *s_flag, int step) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwb = blockDim.x >> 5;
-  const int32_t pos = h.chunk_pos[ci];
-  const int64_t eb = h.chunk_beg[ci], ee = h.chunk_end[ci];
-  const int32_t v = a.members[pos];
-  const bool skip = skipped(a, v);  // block-uniform
-  const uint32_t smask = kHubStageCap - 1;
-  // the staging slots in the order they were first filled (s_flag[0] of them)
-  int32_t *sfill = reinterpret_cast<int32_t *>(svals + kHubStageCap);
-  if (!skip) {
-  for (uint32_t q = threadIdx.x; q < kHubStageCap; q += blockDim.x) { skeys[q] = -1; svals[q] = 0.0; }
-  if (threadIdx.x == 0) { s_self[0] = 0.0; s_flag[0] = 0; }
-  __syncthreads();
-  double sl = warp_accumulate(a, v, eb + 32 * warp, ee, 32 * nwb, skeys, svals, smask, true, sfill,
-                              s_flag);
-  if (lane == 0 && sl != 0.0) atomicAdd(&s_self[0], sl);
-  __syncthreads();
-  const int nfill = s_flag[0];
-  const uint32_t mask = table_cap(a.ptr[v + 1] - a.ptr[v]) - 1;
-  int32_t *keys = h.keys + h.tab_off[pos];
-  double *vals = h.vals + h.tab_off[pos];
-  int32_t *occ = h.occ + h.occ_off[pos];
-  const int32_t own = a.C[v];
-  // Each thread inserts kHubBatch staged keys at once: the probes of one
-  // round are independent CASes in flight together.  Only the filled staging
-  // slots are visited (at most kHubChunk: one round of 4 x 512 keys).
-  for (int q0 = 0; q0 < nfill; q0 += kHubBatch * (int)blockDim.x) {
-    // nfill is the block's: a block-uniform loop
-    int32_t c[kHubBatch];
-    double val[kHubBatch];
-    uint32_t s[kHubBatch];
-    bool pend[kHubBatch], ins[kHubBatch];
-#pragma unroll
-    for (int j = 0; j < kHubBatch; ++j) {
-      const int q = q0 + j * (int)blockDim.x + (int)threadIdx.x;
-      const int32_t sl = (q < nfill) ? sfill[q] : -1;
-      c[j] = (sl >= 0) ? skeys[sl] : -1;
-      val[j] = (sl >= 0) ? svals[sl] : 0.0;
-      pend[j] = c[j] >= 0;
-      ins[j] = false;
-      s[j] = pend[j] ? hash_slot(c[j], mask) : 0u;
-    }
-    bool more = pend[0] || pend[1] || pend[2] || pend[3];
-    while (more) {  // per thread; no warp-synchronous work inside
-      int32_t old[kHubBatch];
-#pragma unroll
-      for (int j = 0; j < kHubBatch; ++j) old[j] = pend[j] ? atomicCAS(&keys[s[j]], -1, c[j]) : 0;
-      more = false;
-#pragma unroll
-      for (int j = 0; j < kHubBatch; ++j) {
-        if (!pend[j]) continue;
-        if (old[j] == -1) { ins[j] = true; pend[j] = false; }
-        else if (old[j] == c[j]) pend[j] = false;
-        else { s[j] = (s[j] + 1) & mask; more = true; }
-      }
-    }
-    // filled-slot list: one counter update per warp
-    int nins = 0;
-#pragma unroll
-    for (int j = 0; j < kHubBatch; ++j) nins += ins[j] ? 1 : 0;
-    int incl = nins;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int y = __shfl_up_sync(FULL, incl, off);
-      if (lane >= off) incl += y;
-    }
-    const int total = __shfl_sync(FULL, incl, 31);
-    int obase = 0;
-    if (lane == 31 && total > 0) obase = atomicAdd(&h.cnt[pos], total);
-    obase = __shfl_sync(FULL, obase, 31) + incl - nins;
-#pragma unroll
-    for (int j = 0; j < kHubBatch; ++j)
-      if (ins[j]) occ[obase++] = (int32_t)s[j];
-#pragma unroll
-    for (int j = 0; j < kHubBatch; ++j) {
-      if (c[j] < 0) continue;
-      atomicAdd(&vals[s[j]], val[j]);
-      if (c[j] == own) atomicAdd(&h.own_w[pos], val[j]);
-    }
-  }
-  if (threadIdx.x == 0 && s_self[0] != 0.0) atomicAdd(&h.self_w[pos], s_self[0]);
-  }  // !skip
-  // The block that finishes a hub's last chunk decides it when the hub has
-  // few distinct communities; otherwise it marks the hub for the segment scan.
-  // Every thread publishes its table and list writes before the countdown.
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_flag[0] = (atomicSub(&h.chunks_left[pos], 1) == 1) ? 1 : 0;
-  __syncthreads();
-  if (!s_flag[0]) return;
-  __threadfence();
-  if (skip) {
-    if (threadIdx.x == 0) {
-      emit_stay(a, pos, v, a.C[v]);
-      h.chunks_left[pos] = (int32_t)((a.ptr[v + 1] - a.ptr[v] + h.chunk - 1) / h.chunk);
-      if (h.epoch) {
-        __threadfence();
-        atomicExch(&h.state[pos], 4u * h.epoch + 1u);
-      }
-    }
-    __syncthreads();
-    return;
-  }
-  const uint32_t mask = table_cap(a.ptr[v + 1] - a.ptr[v]) - 1;
-  int32_t *keys = h.keys + h.tab_off[pos];
-  double *vals = h.vals + h.tab_off[pos];
-  int32_t *occ = h.occ + h.occ_off[pos];
-  const int32_t own = a.C[v];
-  const int32_t nfill = __ldcg(&h.cnt[pos]);
-  if (nfill > kHubInlineCap) {
-    if (threadIdx.x == 0) {
-      if (h.epoch) {
-        atomicExch(&h.state[pos], 4u * h.epoch + 2u);  // its segment tasks decide it
-      } else {
-        h.big[pos] = 1;
-        if (step >= 0) atomicOr(&h.step_big[step], 1);
-      }
-    }
-    __syncthreads();
-    return;
-  }
-  const double degree = a.vDeg[v];
-  const double own_w = __ldcg(&h.own_w[pos]);
-  const double eix = __dsub_rn(own_w, __ldcg(&h.self_w[pos]));
-  const double ax = __dsub_rn(a.cDeg[own], degree);
-  double g = 0.0;
-  int32_t bc = INT32_MAX;
-  hub_scan_slots(a, keys, vals, occ, 0, nfill, own, eix, ax, degree, cst_of(a, v), g, bc);
-  warp_argmax(g, bc);
-  if (lane == 0) { s_g[warp] = g; s_c[warp] = bc; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < nwb; ++k)
-      if (better(s_g[k], s_c[k], g, bc)) { g = s_g[k]; bc = s_c[k]; }
-    emit_decision(a, pos, v, own, finish_choice(a, own, g, bc), degree, own_w, g);
-    h.cnt[pos] = 0;
-    h.self_w[pos] = 0.0;
-    h.own_w[pos] = 0.0;
-    h.chunks_left[pos] = (int32_t)((a.ptr[v + 1] - a.ptr[v] + h.chunk - 1) / h.chunk);
-    if (h.epoch) {
-      __threadfence();
-      atomicExch(&h.state[pos], 4u * h.epoch + 1u);
-    }
-  }
-  __syncthreads();
-}
-
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-constexpr uint32_t kSpinLimit = 1u << 22;  // polls of a segment's wait (x >= 128 ns)
-
-// Persistent kernel: one scan segment of a hub as a block task (all threads
-// call).  Segments are queued after every chunk of their step and a chunk
-// never waits, so the wait ends once the hub's chunks are folded.  The last
-// segment to finish folds the partial arg-maxes and decides the hub.
-__device__ __forceinline__ void hub_segment_task(const SweepArgs &a, const HubWork &h, int64_t si,
-                                                 double *s_g, int32_t *s_c, uint32_t *s_word) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwb = blockDim.x >> 5;
-  const int32_t pos = h.seg_pos[si];
-  const uint32_t decided = 4u * h.epoch + 1u;
-  if (threadIdx.x == 0) {
-    uint32_t st, it = 0;
-    while ((st = ld_acquire(&h.state[pos])) < decided) {
-      if (++it > kSpinLimit) {
-        atomicExch(h.err, 1);
-        st = 0;
-        break;
-      }
-      __nanosleep(128);
-    }
-    s_word[0] = st;
-  }
-  __syncthreads();
-  const uint32_t st = s_word[0];
-  __syncthreads();
-  if (st != decided + 1u) return;  // decided by its last chunk (block-uniform)
-  const int32_t v = a.members[pos];
-  const int32_t own = a.C[v];
-  const double degree = a.vDeg[v];
-  const double own_w = __ldcg(&h.own_w[pos]);
-  const double eix = __dsub_rn(own_w, __ldcg(&h.self_w[pos]));
-  const double ax = __dsub_rn(a.cDeg[own], degree);
-  int32_t *keys = h.keys + h.tab_off[pos];
-  double *vals = h.vals + h.tab_off[pos];
-  const int32_t *occ = h.occ + h.occ_off[pos];
-  const int64_t ob = h.seg_beg[si];
-  const int64_t oe = min(h.seg_end[si], (int64_t)__ldcg(&h.cnt[pos]));
-  double g = 0.0;
-  int32_t bc = INT32_MAX;
-  if (ob < oe) hub_scan_slots(a, keys, vals, occ, ob, oe, own, eix, ax, degree, cst_of(a, v), g, bc);
-  warp_argmax(g, bc);
-  if (lane == 0) { s_g[warp] = g; s_c[warp] = bc; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < nwb; ++k)
-      if (better(s_g[k], s_c[k], g, bc)) { g = s_g[k]; bc = s_c[k]; }
-    h.part_g[si] = g;
-    h.part_c[si] = bc;
-    __threadfence();
-    s_word[0] = (atomicSub(&h.segs_left[pos], 1) == 1) ? 1u : 0u;
-  }
-  __syncthreads();
-  const bool last = s_word[0] != 0;
-  __syncthreads();
-  if (!last || warp != 0) return;
-  __threadfence();
-  g = 0.0;
-  bc = INT32_MAX;
-  for (int64_t k = h.hub_seg_beg[pos] + lane; k < h.hub_seg_end[pos]; k += 32) {
-    const double pg = __ldcg(&h.part_g[k]);
-    const int32_t pc = __ldcg(&h.part_c[k]);
-    if (better(pg, pc, g, bc)) { g = pg; bc = pc; }
-  }
-  warp_argmax(g, bc);
-  if (lane == 0) {
-    emit_decision(a, pos, v, own, finish_choice(a, own, g, bc), degree, own_w, g);
-    h.cnt[pos] = 0;
-    h.self_w[pos] = 0.0;
-    h.own_w[pos] = 0.0;
-    h.chunks_left[pos] = (int32_t)((a.ptr[v + 1] - a.ptr[v] + h.chunk - 1) / h.chunk);
-    h.segs_left[pos] = (int32_t)(h.hub_seg_end[pos] - h.hub_seg_beg[pos]);
-  }
-}
-
-// All threads of the block call; s_g/s_c are 32-entry block scratch.
-__device__ __forceinline__ void hub_scan_segment(const SweepArgs &a, const HubWork &h, int64_t si,
-                                                 double *s_g, int32_t *s_c) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwb = blockDim.x >> 5;
-  const int32_t pos = h.seg_pos[si];
-  if (!h.big[pos]) return;  // decided when its last chunk finished (block-uniform)
-  const int32_t v = a.members[pos];
-  const int32_t own = a.C[v];
-  const double degree = a.vDeg[v];
-  const double eix = __dsub_rn(h.own_w[pos], h.self_w[pos]);
-  const double ax = __dsub_rn(a.cDeg[own], degree);
-  int32_t *keys = h.keys + h.tab_off[pos];
-  double *vals = h.vals + h.tab_off[pos];
-  const int32_t *occ = h.occ + h.occ_off[pos];
-  const int64_t ob = h.seg_beg[si];
-  const int64_t oe = min(h.seg_end[si], (int64_t)h.cnt[pos]);
-  double g = 0.0;
-  int32_t bc = INT32_MAX;
-  hub_scan_slots(a, keys, vals, occ, ob, oe, own, eix, ax, degree, cst_of(a, v), g, bc);
-  warp_argmax(g, bc);
-  if (lane == 0) { s_g[warp] = g; s_c[warp] = bc; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < nwb; ++k)
-      if (better(s_g[k], s_c[k], g, bc)) { g = s_g[k]; bc = s_c[k]; }
-    h.part_g[si] = g;
-    h.part_c[si] = bc;
-  }
-  __syncthreads();
-}
-
-// One warp per hub (all lanes call).
-__device__ __forceinline__ void hub_final(const SweepArgs &a, const HubWork &h, int64_t pos) {
-  const int lane = threadIdx.x & 31;
-  if (!h.big[pos]) return;
-  double g = 0.0;
-  int32_t bc = INT32_MAX;
-  for (int64_t si = h.hub_seg_beg[pos] + lane; si < h.hub_seg_end[pos]; si += 32)
-    if (better(h.part_g[si], h.part_c[si], g, bc)) { g = h.part_g[si]; bc = h.part_c[si]; }
-  warp_argmax(g, bc);
-  if (lane == 0) {
-    const int32_t v = a.members[pos];
-    const int32_t own = a.C[v];
-    emit_decision(a, pos, v, own, finish_choice(a, own, g, bc), a.vDeg[v], h.own_w[pos], g);
-    h.cnt[pos] = 0;
-    h.self_w[pos] = 0.0;
-    h.own_w[pos] = 0.0;
-    h.big[pos] = 0;
-    h.chunks_left[pos] = (int32_t)((a.ptr[v + 1] - a.ptr[v] + h.chunk - 1) / h.chunk);
-  }
-}
 
 // ---------------------------------------------------------------------------
 // Hub rows on thread-block clusters (persistent kernel, parallel modes).  The
@@ -1023,7 +608,7 @@ __device__ __forceinline__ void cluster_accumulate(const SweepArgs &a,
 // sums alternate between two slots by task parity, so rank 0 clears one pair
 // while the blocks may already add to the other.
 __device__ __forceinline__ void cluster_row_tasks(const SweepArgs &a, const HubWork &h, int64_t tb,
-                                               int64_t ntask, int64_t *ctr, int32_t *keys,
+                                               int64_t ntask, unsigned *ctr, int32_t *keys,
                                                double *vals, ClusterShared *cs, double *red,
                                                int32_t *redc) {
   namespace cgx = cooperative_groups;
@@ -1037,7 +622,7 @@ __device__ __forceinline__ void cluster_row_tasks(const SweepArgs &a, const HubW
     vals[q] = 0.0;
   }
   if (rank == 0 && threadIdx.x == 0) {
-    cs->next = (int64_t)atomicAdd((unsigned long long *)ctr, 1ull);
+    cs->next = (int64_t)atomicAdd(ctr, 1u);
     cs->acc[0][0] = cs->acc[0][1] = cs->acc[1][0] = cs->acc[1][1] = 0.0;
   }
   cl.sync();
@@ -1053,7 +638,7 @@ __device__ __forceinline__ void cluster_row_tasks(const SweepArgs &a, const HubW
       if (rank == 0 && threadIdx.x == 0 && part == 0) emit_stay(a, pos, v, own);
       cl.sync();  // every block has read `next`
       if (rank == 0 && threadIdx.x == 0)
-        cs->next = (int64_t)atomicAdd((unsigned long long *)ctr, 1ull);
+        cs->next = (int64_t)atomicAdd(ctr, 1u);
       cl.sync();
       continue;
     }
@@ -1093,7 +678,7 @@ __device__ __forceinline__ void cluster_row_tasks(const SweepArgs &a, const HubW
         if (better(red[k], redc[k], g, bc)) { g = red[k]; bc = redc[k]; }
       cs0->g[rank] = g;
       cs0->c[rank] = bc;
-      if (rank == 0) cs->next = (int64_t)atomicAdd((unsigned long long *)ctr, 1ull);
+      if (rank == 0) cs->next = (int64_t)atomicAdd(ctr, 1u);
     }
     for (uint32_t q = threadIdx.x; q < local; q += blockDim.x) {
       keys[q] = -1;
@@ -1113,7 +698,7 @@ __device__ __forceinline__ void cluster_row_tasks(const SweepArgs &a, const HubW
         h.ct_g[ti] = g;
         h.ct_c[ti] = bc;
         __threadfence();
-        decide = atomicSub(&h.segs_left[pos], 1) == 1;
+        decide = atomicSub(&h.ct_left[ti - part], 1) == 1;
         if (decide) {
           __threadfence();
           const int64_t t0 = ti - part;
@@ -1122,39 +707,12 @@ __device__ __forceinline__ void cluster_row_tasks(const SweepArgs &a, const HubW
             const int32_t pc = __ldcg(&h.ct_c[t0 + k]);
             if (better(pg, pc, g, bc)) { g = pg; bc = pc; }
           }
-          h.segs_left[pos] = (int32_t)nparts;
+          h.ct_left[t0] = (int32_t)nparts;
         }
       }
       if (decide) emit_decision(a, pos, v, own, finish_choice(a, own, g, bc), degree, row_own, g);
     }
   }
-}
-
-__global__ void __launch_bounds__(512) k_hub_accum(SweepArgs a, HubWork h, int64_t cb,
-                                                   int64_t ce) {
-  extern __shared__ unsigned char smem_raw[];
-  __shared__ double s_self[1], s_g[32];
-  __shared__ int32_t s_c[32];
-  __shared__ int s_flag[1];
-  // staging values, the filled-slot list, staging keys (kHubStageSmem bytes)
-  double *svals = reinterpret_cast<double *>(smem_raw);
-  int32_t *skeys = reinterpret_cast<int32_t *>(svals + kHubStageCap) + kHubStageCap;
-  for (int64_t ci = cb + blockIdx.x; ci < ce; ci += gridDim.x)
-    hub_accum_chunk(a, h, ci, skeys, svals, s_self, s_g, s_c, s_flag, -1);
-}
-
-__global__ void __launch_bounds__(256) k_hub_scan(SweepArgs a, HubWork h, int64_t sb,
-                                                  int64_t se) {
-  __shared__ double s_g[32];
-  __shared__ int32_t s_c[32];
-  for (int64_t si = sb + blockIdx.x; si < se; si += gridDim.x) hub_scan_segment(a, h, si, s_g, s_c);
-}
-
-__global__ void __launch_bounds__(256) k_hub_final(SweepArgs a, HubWork h, int64_t b,
-                                                   int64_t e) {
-  const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t pos = b + wid; pos < e; pos += nw) hub_final(a, h, pos);
 }
 
 }  // namespace glv
