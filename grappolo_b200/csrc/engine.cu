@@ -2153,16 +2153,30 @@ int Engine::run_persistent(const Level &L, const std::vector<ClassSched> &sched,
   StepDesc *d_steps = nullptr;
   unsigned *d_ctr = nullptr;
   TRY(alloc(&d_steps, steps.size()));
-  TRY(alloc(&d_ctr, 3 * steps.size()));  // block, team and cluster queues of every step
+  const int nclass = (int)cls_b.size(), nsteps = (int)steps.size();
+  // block, team and cluster queues of every step, then the classes' moved flags
+  const size_t nctr = 3 * steps.size() + cls_b.size();
+  TRY(alloc(&d_ctr, nctr));
   TRY(upload(s_, d_steps, steps));
-  int64_t *d_cls_b = nullptr;
-  int32_t *d_kept = nullptr;
-  const int nclass = (int)cls_b.size();
+  int64_t *d_step_b = nullptr;
+  int32_t *d_kept = nullptr, *d_step_cls = nullptr;
   const int64_t nmem = cls_e.empty() ? 0 : cls_e.back();
   Batch *bt = bt_;
   if ((!jacobi && learned()) || bt) {
-    TRY(alloc(&d_cls_b, nclass)); TRY(alloc(&d_kept, nclass));
-    TRY(upload(s_, d_cls_b, cls_b));
+    std::vector<int64_t> step_b(nsteps);
+    std::vector<int32_t> ends(2 * (size_t)nsteps);  // each step's class: first, then last step
+    for (int k = 0; k < nsteps; ++k) {
+      step_b[k] = steps[k].seg[0];
+      ends[k] = (k > 0 && steps[k - 1].cls == steps[k].cls) ? ends[k - 1] : k;
+    }
+    for (int k = nsteps - 1; k >= 0; --k)
+      ends[nsteps + k] =
+          (k + 1 < nsteps && steps[k + 1].cls == steps[k].cls) ? ends[nsteps + k + 1] : k;
+    TRY(alloc(&d_step_b, nsteps)); TRY(alloc(&d_kept, nsteps));
+    TRY(alloc(&d_step_cls, 2 * (size_t)nsteps));
+    TRY(upload(s_, d_step_b, step_b));
+    TRY(upload(s_, d_step_cls, ends));
+    CK(cudaStreamSynchronize(s_));
   }
   if (bt) {
     if (!skip_) TRY(alloc(&skip_, nv0_ + 1));
@@ -2185,6 +2199,7 @@ int Engine::run_persistent(const Level &L, const std::vector<ClassSched> &sched,
   p.cDeg = cDeg;
   p.cSize = cSize;
   p.task_ctr = d_ctr;
+  p.moved = reinterpret_cast<int *>(d_ctr + 3 * steps.size());
   p.nnz = L.nnz;
   p.split_row = split_row_;
   // Fast mode on non-integral weights (no exact result to keep): after the
@@ -2328,29 +2343,29 @@ int Engine::run_persistent(const Level &L, const std::vector<ClassSched> &sched,
         LAUNCH(k_gate_infer, std::max(1, (int)std::min<int64_t>((L.nv + 127) / 128, nsm_ * 8)), 256, 0,
                s_, L.nv, tracing ? (const float *)feat_ : nullptr, fsrc, gate_p_, tau, L.ptr,
                (float *)nullptr, skip_, evald_);
-        CK(cudaMemsetAsync(d_kept, 0, nclass * sizeof(int32_t), s_));
-        LAUNCH(k_class_kept, grid_for(nmem, 256, nsm_ * 8), 256, 0, s_, nclass, d_cls_b, nmem,
-               members_, skip_, d_kept);
+        CK(cudaMemsetAsync(d_kept, 0, nsteps * sizeof(int32_t), s_));
+        LAUNCH(k_steps_kept, grid_for(nmem, 256, nsm_ * 8), 256, 0, s_, nsteps, d_step_b,
+               d_step_cls, d_step_cls + nsteps, 1, nmem, members_, skip_, d_kept);
         p.a.skip = skip_;
       }
-      p.class_kept = gated_now ? d_kept : nullptr;
+      p.kept = gated_now ? d_kept : nullptr;
     }
     double batch_edges = 0;
     if (bt) {
       // graphs that have converged (or sit out this phase) are skipped whole
       LAUNCH(k_graph_skip, grid_for(L.nv, 256, nsm_ * 16), 256, 0, s_, L.nv, bt->gid, bt->act,
              skip_);
-      CK(cudaMemsetAsync(d_kept, 0, nclass * sizeof(int32_t), s_));
-      LAUNCH(k_class_kept, grid_for(nmem, 256, nsm_ * 8), 256, 0, s_, nclass, d_cls_b, nmem,
-             members_, skip_, d_kept);
+      CK(cudaMemsetAsync(d_kept, 0, nsteps * sizeof(int32_t), s_));
+      LAUNCH(k_steps_kept, grid_for(nmem, 256, nsm_ * 8), 256, 0, s_, nsteps, d_step_b,
+             d_step_cls, d_step_cls + nsteps, 0, nmem, members_, skip_, d_kept);
       CK(cudaMemsetAsync(bt->gacc, 0, 2 * bt->G * sizeof(double), s_));
       p.a.skip = skip_;
-      p.class_kept = d_kept;
+      p.kept = d_kept;
       for (int g = 0; g < bt->G; ++g)
         if (bt->h_act[g]) batch_edges += (double)bt->gnnz[g];
     }
     p.exx_mode = (carry_exx && n >= 2) ? (check_exx ? 2 : 1) : 0;
-    cudaError_t e = cudaMemsetAsync(d_ctr, 0, 3 * steps.size() * sizeof(unsigned), s_);
+    cudaError_t e = cudaMemsetAsync(d_ctr, 0, nctr * sizeof(unsigned), s_);
     p.h.epoch = ++epoch_;
     if (e0) cudaEventRecord(e0, s_);
     if (e == cudaSuccess && cl > 0) {
@@ -2542,7 +2557,8 @@ int Engine::run_persistent(const Level &L, const std::vector<ClassSched> &sched,
   dfree(d_trace);
   dfree(d_ctr);
   dfree(pair_u); dfree(pair_t); dfree(pair_w);
-  dfree(d_cls_b);
+  dfree(d_step_b);
+  dfree(d_step_cls);
   dfree(d_kept);
   dfree(exx_buf);
   if (e0) cudaEventDestroy(e0);

@@ -182,8 +182,8 @@ __device__ __forceinline__ void hub_chunk_task(const SweepArgs &a, const HubWork
     for (int q = threadIdx.x; q <= hb.nparts; q += kHubThreads) sh->hist[q] = 0;
     double self_w = 0.0, own_w = 0.0;
     const int rounds =
-        row_accumulate<kHubThreads>(a, v, a.C[v], ch.beg, ch.beg + ch.len, keys, vals,
-                                    kHubTableCap - 1, fill + threadIdx.x, self_w, own_w);
+        row_accumulate<kHubThreads>(a, v, a.C[v], ch.beg, ch.len, keys, vals, kHubTableCap - 1,
+                                    fill + threadIdx.x, self_w, own_w);
     if (__any_sync(FULL, self_w != 0.0)) self_w = warp_sum(self_w);
     if (__any_sync(FULL, own_w != 0.0)) own_w = warp_sum(own_w);
     if (lane == 0) {

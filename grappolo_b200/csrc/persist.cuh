@@ -55,7 +55,8 @@ struct IterArgs {
   int32_t *cSize;
   uint64_t *trace;         // optional: globaltimer at each barrier, 4 per step + 2
   unsigned *task_ctr;      // per step: next block, team and cluster task (zero at launch)
-  const int32_t *class_kept;  // gated sweeps: vertices the gate kept per class (NULL = all)
+  int *moved;              // per colour class: some vertex moved (zero at launch)
+  const int32_t *kept;     // gated or batched sweeps: k_steps_kept's flags (NULL = all steps run)
   int64_t nnz;
   const int64_t *split_row;   // merge-path tile boundaries of the level
   // batches of graphs: per-graph modularity sums instead of one Q
@@ -77,20 +78,26 @@ struct IterArgs {
   int64_t npairs;
 };
 
-// Gated or batched sweeps: kept[c] = 1 when some member of colour class c is
-// evaluated (kept must be zero on entry).  Member positions are strided over
-// the grid; a position's class is found by binary search in cls_begin.
-__global__ void k_class_kept(int nclass, const int64_t *cls_begin, int64_t nmem,
+// Gated or batched sweeps: kept[s] & 2 when some member of step s is evaluated,
+// kept[s] & 1 at the last step of a class when some member of the class is
+// (kept must be zero on entry).  With per_class a class runs all its steps or
+// none.  Member positions are strided over the grid; a position's step is found
+// by binary search in step_begin; [step_first, step_last] are its class's.
+__global__ void k_steps_kept(int nsteps, const int64_t *step_begin, const int32_t *step_first,
+                             const int32_t *step_last, int per_class, int64_t nmem,
                              const int32_t *members, const uint8_t *skip, int32_t *kept) {
   for (int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; pos < nmem;
        pos += (int64_t)gridDim.x * blockDim.x) {
     if (skip[members[pos]]) continue;
-    int lo = 0, hi = nclass - 1;  // last class starting at or before pos
+    int lo = 0, hi = nsteps - 1;  // last step starting at or before pos
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      if (cls_begin[mid] <= pos) lo = mid; else hi = mid - 1;
+      if (step_begin[mid] <= pos) lo = mid; else hi = mid - 1;
     }
-    if (kept[lo] == 0) kept[lo] = 1;
+    const int last = step_last[lo];
+    for (int q = per_class ? step_first[lo] : lo; q <= (per_class ? last : lo); ++q)
+      if (!(kept[q] & 2)) atomicOr(&kept[q], 2);
+    if (!(kept[last] & 1)) atomicOr(&kept[last], 1);
   }
 }
 
@@ -142,25 +149,30 @@ static_assert(kPersistFill / (kPersistThreads / kTeamThreads) >= 1024 && 127 < 4
               "every entry of a row has a filled-slot entry");
 
 // Community totals += the deltas the sweep accumulated (see k_apply_deltas).
-__device__ __forceinline__ void apply_deltas_range(const IterArgs &p, int64_t b, int64_t e,
-                                                   int64_t gt, int64_t ngt) {
-  for (int64_t pos = b + gt; pos < e; pos += ngt) {
-    const int32_t o = p.a.move_old[pos];
+// The whole stage sits between two grid barriers, so what counts is its chain
+// of dependent accesses: a position's records load together, and both
+// communities' claims and totals are in flight together (one claim at a time,
+// each an L2 round trip, took 4.3 us a step on R-MAT 20's second level; now
+// 2.2).  Only the thread that claimed a nonzero delta writes a total, and
+// stage 1 is over, so a total read beside the claim is still current.
+__device__ __forceinline__ void apply_deltas_range(const IterArgs &p, int b, int e, int gt,
+                                                   int ngt) {
+  for (int pos = b + gt; pos < e; pos += ngt) {
+    const int32_t o = p.a.move_old[pos], n = p.a.move_new[pos];
     if (p.a.defer_c) {
       // deferred decisions: moves, and isolated vertices leaving every community
-      const int32_t n = p.a.move_new[pos];
       if (o >= 0 || n < 0) p.a.C[p.a.members[pos]] = n;
     }
     if (o < 0) continue;
-    const int32_t cs[2] = {p.a.move_new[pos], o};
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int32_t c = cs[k];
-      const unsigned long long bits = atomicExch((unsigned long long *)&p.a.dDeg[c], 0ull);
-      if (bits != 0ull) p.cDeg[c] = __dadd_rn(p.cDeg[c], __longlong_as_double((long long)bits));
-      const int32_t s = atomicExch(&p.a.dSize[c], 0);
-      if (s != 0) p.cSize[c] += s;
-    }
+    const unsigned long long dn = atomicExch((unsigned long long *)&p.a.dDeg[n], 0ull);
+    const unsigned long long od = atomicExch((unsigned long long *)&p.a.dDeg[o], 0ull);
+    const int32_t sn = atomicExch(&p.a.dSize[n], 0), so = atomicExch(&p.a.dSize[o], 0);
+    const double cn = __ldcg(&p.cDeg[n]), co = __ldcg(&p.cDeg[o]);
+    const int32_t zn = __ldcg(&p.cSize[n]), zo = __ldcg(&p.cSize[o]);
+    if (dn) p.cDeg[n] = __dadd_rn(cn, __longlong_as_double((long long)dn));
+    if (od) p.cDeg[o] = __dadd_rn(co, __longlong_as_double((long long)od));
+    if (sn) p.cSize[n] = zn + sn;
+    if (so) p.cSize[o] = zo + so;
   }
 }
 
@@ -192,6 +204,14 @@ __device__ __forceinline__ void modularity_fold(const IterArgs &p, int64_t npart
   }
 }
 
+// threadIdx.x read anew: indexes derived from it are not kept (and spilled)
+// across a step's tasks, whose reloads after a grid barrier miss in L1.
+__device__ __forceinline__ int thread_id() {
+  int t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
+}
+
 // kClusters: the instantiation launched with a cluster dimension, which runs
 // the steps' cluster tasks; the other one leaves that code out entirely (its
 // registers go to the other paths).
@@ -201,25 +221,13 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_sweep_iteration(IterArgs
   extern __shared__ unsigned char smem_raw[];
   __shared__ double s_self[32], s_own[32], s_g[32], sh[32];
   __shared__ int32_t s_c[32];
-  const int warp = threadIdx.x >> 5, nwb = blockDim.x >> 5;
-  const int ngw = gridDim.x * nwb;
-  // warps numbered across blocks first: a step with few warp items spreads over SMs
-  const int gwi = warp * gridDim.x + blockIdx.x;
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t ngt = (int64_t)gridDim.x * blockDim.x;
   // shared table region: one 8192-slot table (block tasks), four 2048-slot
-  // team tables, or a 256-slot table per warp inside its team's table
-  const int team = threadIdx.x / kTeamThreads, tt = threadIdx.x % kTeamThreads;
-  double *tvals = reinterpret_cast<double *>(smem_raw);
-  int32_t *tkeys = reinterpret_cast<int32_t *>(tvals + kPersistTableCap);
-  double *team_vals = tvals + (size_t)team * kTeamCap;
-  int32_t *team_keys = tkeys + (size_t)team * kTeamCap;
-  double *wvals = team_vals + (size_t)(tt >> 5) * kPersistWarpCap;
-  int32_t *wkeys = team_keys + (size_t)(tt >> 5) * kPersistWarpCap;
-  // filled slots: the block's, a quarter of it per team, 128 of that per warp
-  uint16_t *fill = reinterpret_cast<uint16_t *>(smem_raw + kPersistTableBytes);
-  uint16_t *team_fill = fill + (size_t)team * (kPersistFill * kTeamThreads / kPersistThreads);
-  uint16_t *wfill = team_fill + (size_t)(tt >> 5) * 128;
+  // team tables, or a 256-slot table per warp inside its team's table; the
+  // filled slots likewise: the block's, a quarter of it per team, 128 of that
+  // per warp
+  double *const tvals = reinterpret_cast<double *>(smem_raw);
+  int32_t *const tkeys = reinterpret_cast<int32_t *>(tvals + kPersistTableCap);
+  uint16_t *const fill = reinterpret_cast<uint16_t *>(smem_raw + kPersistTableBytes);
   // tables are empty between tasks; every task empties the slots it filled
   for (int q = threadIdx.x; q < kPersistTableCap; q += kPersistThreads) {
     tkeys[q] = -1;
@@ -237,22 +245,28 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_sweep_iteration(IterArgs
   if (p.a.exx_delta && threadIdx.x == 0) p.a.exx_delta[blockIdx.x] = 0.0;
   // The step's description in shared memory, loaded a step ahead: its values
   // cost no registers across the tasks and no L2 round trip after a barrier.
-  __shared__ StepDesc s_step[2];
+  // Three of them, so that a step's may be read until the next step's barrier.
+  __shared__ StepDesc s_step[3];
+  __shared__ int s_keep[3];
   if (threadIdx.x < kStepWords && p.nsteps > 0)
     reinterpret_cast<int32_t *>(&s_step[0])[threadIdx.x] =
         reinterpret_cast<const int32_t *>(&p.steps[0])[threadIdx.x];
+  if (threadIdx.x == kStepWords && p.nsteps > 0) s_keep[0] = p.kept ? p.kept[0] : 3;
+  if (threadIdx.x == 0) block_moved() = 0;
   __syncthreads();
-  for (int s = 0; s < p.nsteps; ++s) {
-    const StepDesc &st = s_step[s & 1];
-    // (read after this step's barriers, or after the one below for a skipped step)
-    if (threadIdx.x < kStepWords && s + 1 < p.nsteps)
-      reinterpret_cast<int32_t *>(&s_step[(s + 1) & 1])[threadIdx.x] =
-          reinterpret_cast<const int32_t *>(&p.steps[s + 1])[threadIdx.x];
-    // a class the gate emptied is skipped whole (no work, no grid barrier)
-    if (p.class_kept && p.class_kept[st.cls] == 0) {
-      __syncthreads();
-      continue;
+  for (int s = 0, cur = 0; s < p.nsteps; ++s, cur = (cur == 2) ? 0 : cur + 1) {
+    const StepDesc &st = s_step[cur];
+    {
+      const int nx = (cur == 2) ? 0 : cur + 1, t = thread_id();
+      if (t < kStepWords && s + 1 < p.nsteps)
+        reinterpret_cast<int32_t *>(&s_step[nx])[t] =
+            reinterpret_cast<const int32_t *>(&p.steps[s + 1])[t];
+      if (t == kStepWords && s + 1 < p.nsteps) s_keep[nx] = p.kept ? p.kept[s + 1] : 3;
     }
+    // a step with nothing to evaluate is skipped (no work, no grid barrier)
+    if (!(s_keep[cur] & 2)) {
+      __syncthreads();
+    } else {
     // Stage 1 in three parts, each from its own queue: (A) hub chunks and
     // rows of 1024..4095 entries, whole blocks with an 8192-slot table;
     // (B) rows of 128..1023 entries, 128-thread teams (four per block, each
@@ -275,14 +289,14 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_sweep_iteration(IterArgs
       // hub chunks, then block rows, then hub partitions (which wait for
       // their hub's chunks: every chunk is handed out before any partition)
       unsigned *ctr = &p.task_ctr[3 * s];
-      if (threadIdx.x == 0) s_task[0] = (int)atomicAdd(ctr, 1u);
+      if (thread_id() == 0) s_task[0] = (int)atomicAdd(ctr, 1u);
       __syncthreads();
       for (unsigned it = 0;; ++it) {
         int t = s_task[it & 1];
         if (t >= st.hub_chunk[1] - st.hub_chunk[0] + st.seg[BIN_BLOCK + 1] - st.seg[BIN_BLOCK] +
                      st.hub_segs[1] - st.hub_segs[0])
           break;
-        const int nxt = (threadIdx.x == 0) ? (int)atomicAdd(&p.task_ctr[3 * s], 1u) : 0;
+        const int nxt = (thread_id() == 0) ? (int)atomicAdd(&p.task_ctr[3 * s], 1u) : 0;
         if (t < st.hub_chunk[1] - st.hub_chunk[0]) {
           hub_chunk_task(p.a, p.h, st.hub_chunk[0] + t, tkeys, tvals, fill, &s_hub, s_g, s_c);
         } else {
@@ -295,12 +309,13 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_sweep_iteration(IterArgs
             hub_part_task(p.a, p.h, st.hub_segs[0] + (t - nblk), tkeys, tvals, fill, &s_hub, s_g,
                           s_c);
         }
-        if (threadIdx.x == 0) s_task[(it + 1) & 1] = nxt;
+        if (thread_id() == 0) s_task[(it + 1) & 1] = nxt;
         __syncthreads();
       }
       GLV_QTRACE(s, 0, threadIdx.x == 0);
     }
     if (st.seg[BIN_T256 + 1] > st.seg[BIN_T128]) {
+      const int team = thread_id() / kTeamThreads, tt = thread_id() % kTeamThreads;
       if (tt == 0) s_team_task[team][0] = (int)atomicAdd(&p.task_ctr[3 * s + 1], 1u);
       team_sync<128>(team);
       for (unsigned it = 0;; ++it) {
@@ -310,14 +325,18 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_sweep_iteration(IterArgs
         if (t >= st.seg[BIN_T256 + 1] - st.seg[BIN_T128]) break;
         const int nxt = (tt == 0) ? (int)atomicAdd(&p.task_ctr[3 * s + 1], 1u) : 0;
         const int pos = (t < n256) ? st.seg[BIN_T256] + t : st.seg[BIN_T128] + (t - n256);
-        row_vertex<128>(p.a, pos, team_keys, team_vals, team_fill, team, s_self + 4 * team,
-                        s_own + 4 * team, s_g + 4 * team, s_c + 4 * team);
+        row_vertex<128>(p.a, pos, tkeys + team * kTeamCap, tvals + team * kTeamCap,
+                        fill + team * (kPersistFill * kTeamThreads / kPersistThreads), team,
+                        s_self + 4 * team, s_own + 4 * team, s_g + 4 * team, s_c + 4 * team);
         if (tt == 0) s_team_task[team][(it + 1) & 1] = nxt;
         team_sync<128>(team);
       }
       GLV_QTRACE(s, 1, tt == 0);
     }
     {
+      // warps numbered across blocks first: a step with few warp items spreads over SMs
+      const int warp = thread_id() >> 5, ngw = gridDim.x * (kPersistThreads / 32);
+      const int gwi = warp * gridDim.x + blockIdx.x;
       const int i4 = (st.seg[1] - st.seg[0] + 7) / 8, i8 = (st.seg[2] - st.seg[1] + 3) / 4;
       const int i16 = (st.seg[3] - st.seg[2] + 1) / 2;
       const int witems = i4 + i8 + i16 + st.seg[5] - st.seg[3];
@@ -331,20 +350,34 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_sweep_iteration(IterArgs
         q -= i16 - st.seg[3];  // its member position
         if (q < st.seg[4]) small_item<32>(p.a, q, st.seg[4]);
         else
-          row_vertex<32>(p.a, q, wkeys, wvals, wfill, 0, nullptr, nullptr, nullptr, nullptr);
+          row_vertex<32>(p.a, q,
+                         tkeys + (warp >> 2) * kTeamCap + (warp & 3) * kPersistWarpCap,
+                         tvals + (warp >> 2) * kTeamCap + (warp & 3) * kPersistWarpCap,
+                         fill + (warp >> 2) * (kPersistFill * kTeamThreads / kPersistThreads) +
+                             (warp & 3) * 128,
+                         0, nullptr, nullptr, nullptr, nullptr);
       }
       GLV_QTRACE(s, 2, (threadIdx.x & 31) == 0 && gwi < witems);
     }
-    // read before the barrier: past it another warp may load over this step
-    const int apply_b = st.apply[0], apply_e = st.apply[1];
+    __syncthreads();
+    if (thread_id() == 0 && block_moved()) {
+      p.moved[st.cls] = 1;
+      block_moved() = 0;
+    }
     grid.sync();
     GLV_TRACE(4 * s);
-    if (!p.jacobi && apply_e > apply_b) {
-      apply_deltas_range(p, apply_b, apply_e, gt, ngt);
+    }
+    // A class that moved nothing has no totals to update (in a phase's first
+    // sweep the apply stage also takes isolated vertices out of C).
+    if (!p.jacobi && st.apply[1] > st.apply[0] && (s_keep[cur] & 1) &&
+        (p.a.iter <= 1 || __ldcg(&p.moved[st.cls]))) {
+      apply_deltas_range(p, st.apply[0], st.apply[1], blockIdx.x * kPersistThreads + thread_id(),
+                         gridDim.x * kPersistThreads);
       grid.sync();
       GLV_TRACE(4 * s + 3);
     }
   }
+  const int gt = blockIdx.x * kPersistThreads + threadIdx.x, ngt = gridDim.x * kPersistThreads;
   {
     // merge-path tiles, one partial pair per block
     double ex = 0.0, a2 = 0.0;

@@ -35,6 +35,10 @@ __device__ __forceinline__ void team_sync(int team) {
   else asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(T) : "memory");
 }
 
+__device__ __forceinline__ void prefetch_l1(const void *p) {
+  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
 // Sums x over the lanes of each group (m: the lanes with this lane's key);
 // the group's lowest lane holds the group's sum.
 __device__ __forceinline__ double group_sum(double x, unsigned m) {
@@ -59,65 +63,62 @@ __device__ __forceinline__ double warp_sum(double x) {
   return x;
 }
 
-// Adds the entries [rb, re) of v's row to the table, T at a time.  Entries of
-// the row's own community go to own_w, self-loops to self_w (both per lane).
-// fill[r * T] is this thread's slot of round r (kNoSlot: none filled).
-// Returns the rounds of this warp.
+// Adds the `len` entries from rb on (of v's row) to the table, T at a time.
+// Entries of the row's own community go to own_w, self-loops to self_w (both
+// per lane).  fill[r * T] is this thread's slot of round r (kNoSlot: none
+// filled).  Returns the rounds of this warp.
 template <int T>
 __device__ __forceinline__ int row_accumulate(const SweepArgs &a, int32_t v, int32_t own,
-                                              int64_t rb, int64_t re, int32_t *keys, double *vals,
+                                              int64_t rb, int len, int32_t *keys, double *vals,
                                               uint32_t mask, uint16_t *fill, double &self_w,
                                               double &own_w) {
   const int tt = threadIdx.x % T, lane = threadIdx.x & 31;
+  const int32_t *const tail = a.tail + rb;
+  const double *const w = a.w + rb;
   // Software pipeline, two rounds deep: while this round is folded, the next
   // round's communities are gathered and the round after's entries load.
   // Neighbours' communities do not change during the sweep of one step.  The
   // entries are read once per sweep: streaming loads keep them from pushing the
   // gathered per-vertex arrays out of L2.
-  const int64_t j0 = rb + tt, j1 = j0 + T;
-  int32_t t_cur = (j0 < re) ? __ldcs(&a.tail[j0]) : -1;
-  double w_cur = (j0 < re) ? __ldcs(&a.w[j0]) : 0.0;
-  int32_t t_next = (j1 < re) ? __ldcs(&a.tail[j1]) : -1;
-  double w_next = (j1 < re) ? __ldcs(&a.w[j1]) : 0.0;
-  int32_t c_cur = (j0 < re) ? a.C[t_cur] : -1;
+  int32_t t_cur = (tt < len) ? __ldcs(tail + tt) : -1;
+  double w_cur = (tt < len) ? __ldcs(w + tt) : 0.0;
+  int32_t t_next = (tt + T < len) ? __ldcs(tail + tt + T) : -1;
+  double w_next = (tt + T < len) ? __ldcs(w + tt + T) : 0.0;
+  int32_t c_cur = (tt < len) ? a.C[t_cur] : -1;
   bool group = true;  // the row repeats communities: group a round's equal ones
   int r = 0;
-  for (int64_t base = rb + (tt - lane); base < re; base += T, ++r) {
-    const int64_t j = base + lane;
-    const bool has = j < re;
+  for (int j = tt; j - lane < len; j += T, ++r) {
     const int32_t t = t_cur, c = c_cur;
     const double wt = w_cur;
-    const int64_t jn = j + T, jnn = j + 2 * T;
-    c_cur = (jn < re) ? a.C[t_next] : -1;
+    c_cur = (j + T < len) ? a.C[t_next] : -1;
     t_cur = t_next;
     w_cur = w_next;
-    t_next = (jnn < re) ? __ldcs(&a.tail[jnn]) : -1;
-    w_next = (jnn < re) ? __ldcs(&a.w[jnn]) : 0.0;
-    if (has && t == v) self_w = __dadd_rn(self_w, wt);
-    if (has && c == own) own_w = __dadd_rn(own_w, wt);
-    const bool act = has && c != own;
-    const int n = __popc(__ballot_sync(FULL, act));
-    bool put = act;
+    t_next = (j + 2 * T < len) ? __ldcs(tail + j + 2 * T) : -1;
+    w_next = (j + 2 * T < len) ? __ldcs(w + j + 2 * T) : 0.0;
+    if (t == v) self_w = __dadd_rn(self_w, wt);
+    if (c == own) own_w = __dadd_rn(own_w, wt);
+    bool put = j < len && c != own;
+    const int n = __popc(__ballot_sync(FULL, put));
     double x = wt;
     const bool grouped = group;
     if (group) {
-      const unsigned m = __match_any_sync(FULL, act ? c : -1);
-      put = act && lane == __ffs(m) - 1;
-      x = group_sum(wt, act ? m : 0u);
+      const unsigned m = __match_any_sync(FULL, put ? c : -1);
+      x = group_sum(wt, put ? m : 0u);
+      put = put && lane == __ffs(m) - 1;
       group = 4 * __popc(__ballot_sync(FULL, put)) <= 3 * n;
     }
-    uint16_t slot = kNoSlot;
+    uint32_t slot = kNoSlot;
     if (put) {
       uint32_t s = hash_slot(c, mask);
       while (true) {
         const int32_t k = atomicCAS(&keys[s], -1, c);
-        if (k == -1) slot = (uint16_t)s;
+        if (k == -1) slot = s;
         if (k == -1 || k == c) break;
         s = (s + 1) & mask;
       }
       atomicAdd(&vals[s], x);
     }
-    fill[r * T] = slot;
+    fill[r * T] = (uint16_t)slot;
     if (!grouped) group = 2 * __popc(__ballot_sync(FULL, slot != kNoSlot)) < n;
   }
   return r;
@@ -169,16 +170,19 @@ __device__ __forceinline__ void row_vertex(const SweepArgs &a, int64_t pos, int3
     if (tt == 0) emit_stay(a, pos, v, a.C[v]);
     return;
   }
-  // the row's bounds and the vertex's own values load together, the totals of
-  // its community right after: they arrive while the row accumulates
-  const int64_t rb = a.ptr[v], re = a.ptr[v + 1];
+  const int64_t rb = a.ptr[v];
+  const int len = (int)(a.ptr[v + 1] - rb);
   const int32_t own = a.C[v];
+  // the vertex's and its community's totals come into L1 while the row
+  // accumulates (no registers held for them)
+  prefetch_l1(&a.vDeg[v]);
+  prefetch_l1(&a.cDeg[own]);
+  if (tt == 0) prefetch_l1(&a.cSize[own]);
+  double self_w = 0.0, own_w = 0.0;
+  const int rounds = row_accumulate<T>(a, v, own, rb, len, keys, vals, table_cap(len) - 1,
+                                       fill + tt, self_w, own_w);
   const double degree = a.vDeg[v];
   const double cdeg_own = a.cDeg[own];
-  const int32_t own_size = (tt == 0) ? a.cSize[own] : 0;
-  double self_w = 0.0, own_w = 0.0;
-  const int rounds = row_accumulate<T>(a, v, own, rb, re, keys, vals, table_cap(re - rb) - 1,
-                                       fill + tt, self_w, own_w);
   if (__any_sync(FULL, self_w != 0.0)) self_w = warp_sum(self_w);
   if (__any_sync(FULL, own_w != 0.0)) own_w = warp_sum(own_w);
   if (NW > 1) {
@@ -205,7 +209,7 @@ __device__ __forceinline__ void row_vertex(const SweepArgs &a, int64_t pos, int3
   if (tt == 0) {
     for (int k = 1; k < NW; ++k)
       if (better(s_g[k], s_c[k], g, bc)) { g = s_g[k]; bc = s_c[k]; }
-    emit_decision(a, pos, v, own, finish_choice(a, own, own_size, g, bc), degree, own_w, g);
+    emit_decision(a, pos, v, own, finish_choice(a, own, a.cSize[own], g, bc), degree, own_w, g);
   }
   if (NW == 1) __syncwarp();
 }

@@ -66,6 +66,13 @@ __device__ __forceinline__ double cst_of(const SweepArgs &a, int32_t v) {
   return a.gid ? a.gcst[a.gid[v]] : a.constant;
 }
 
+// Set when a vertex that this block decided moves (read and cleared by the
+// persistent kernel at the end of a step).
+__device__ __forceinline__ int &block_moved() {
+  __shared__ int moved;
+  return moved;
+}
+
 // A vertex the gate left out keeps its community and moves nothing.
 __device__ __forceinline__ void emit_stay(const SweepArgs &a, int64_t pos, int32_t v,
                                           int32_t own) {
@@ -101,6 +108,7 @@ __device__ __forceinline__ void emit_decision(const SweepArgs &a, int64_t pos, i
   }
   if (moved && a.last_move) a.last_move[v] = a.iter;
   if (moved && a.atomic_deltas) {
+    block_moved() = 1;
     atomicAdd(&a.dDeg[target], degree);
     atomicAdd(&a.dDeg[own], -degree);
     atomicAdd(&a.dSize[target], 1);
