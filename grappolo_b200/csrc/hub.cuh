@@ -27,9 +27,11 @@ constexpr int kHubTableCap = 8192;   // the block's table
 constexpr int kHubList = 4096;       // filled slots a merge may hold at once
 constexpr int kHubInline = 2048;     // pairs the last chunk's block merges itself
 constexpr int kHubMaxParts = 512;
-constexpr int kHubPartEntries = 2048;  // row entries per partition (more only past kHubMaxParts)
+constexpr int kHubPartEntries = 1024;  // row entries per partition (more only past kHubMaxParts)
+constexpr int kHubRuns = 512;        // chunks a merge looks up at a time
 constexpr uint32_t kSpinLimit = 1u << 22;  // polls of a partition's wait (>= 128 ns each)
 static_assert(kHubChunk <= 2048 && kHubChunk <= kHubTableCap / 2, "a chunk fits the table");
+static_assert(kHubRuns <= kHubThreads && kHubRuns <= kHubMaxParts, "one thread per run");
 static_assert(kHubChunk < 65536 && kHubTableCap <= kNoSlot, "16-bit offsets and slots");
 
 // Partitions of a row (a power of two, at least 2).
@@ -41,7 +43,9 @@ __host__ __device__ inline int hub_parts(int64_t deg) {
 
 // Block scratch of the hub tasks.
 struct HubShared {
-  int hist[kHubMaxParts + 1];  // pairs per partition, then running offsets
+  int hist[kHubMaxParts + 1];  // pairs per partition, then running offsets; merge: run starts
+  int base[kHubRuns];          // merge: the runs' first pairs, from the hub's first
+  int wsum[kHubThreads / 32];
   int count;                   // merge: filled slots listed
   int over;                    // merge: more distinct communities than the list holds
   int flag;
@@ -66,30 +70,59 @@ __device__ __forceinline__ void hub_merge(const SweepArgs &a, const HubWork &h, 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int NW = kHubThreads / 32;
   const uint32_t mask = kHubTableCap - 1;
+  const int64_t out0 = h.chunks[hb.chunk0].out;
   int bits = 0;
   for (uint32_t share = 0; share < (1u << bits);) {
     if (threadIdx.x == 0) { sh->count = 0; sh->over = 0; }
     __syncthreads();
     const uint32_t smask = (1u << bits) - 1u;
-    for (int k = warp; k < hb.nchunks; k += NW) {
-      const HubChunk &ch = h.chunks[hb.chunk0 + k];
-      const int64_t out = ch.out;
-      const uint16_t *off = h.part_off + ch.off;
-      const int b = __ldcg(&off[p0]), e = __ldcg(&off[p1]);
-      for (int i = b + lane; i - lane < e; i += 32) {
-        const bool has = i < e;
-        const int32_t c = has ? __ldcg(&h.out_c[out + i]) : -1;
-        const double w = has ? __ldcg(&h.out_w[out + i]) : 0.0;
-        const bool mine = has && ((mix32((uint32_t)c) >> 12) & smask) == share;
+    // The chunks' runs of these partitions as one sequence, kHubRuns chunks at
+    // a time: every thread looks one chunk up, then all threads share the pairs
+    // (a warp per chunk left most lanes idle: runs are short and few).
+    for (int k0 = 0; k0 < hb.nchunks; k0 += kHubRuns) {
+      const int nk = min(kHubRuns, hb.nchunks - k0);
+      int mine = 0;
+      if (threadIdx.x < nk) {
+        const HubChunk &ch = h.chunks[hb.chunk0 + k0 + threadIdx.x];
+        const uint16_t *off = h.part_off + ch.off;
+        const int b = __ldcg(&off[p0]);
+        mine = __ldcg(&off[p1]) - b;
+        sh->base[threadIdx.x] = (int)(ch.out - out0) + b;
+      }
+      // exclusive prefix of the run lengths: within the warp, then over warps
+      int incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) sh->wsum[warp] = incl;
+      __syncthreads();
+      int before = 0, total = 0;
+#pragma unroll
+      for (int q = 0; q < NW; ++q) {
+        before += q < warp ? sh->wsum[q] : 0;
+        total += sh->wsum[q];
+      }
+      if (threadIdx.x < nk) sh->hist[threadIdx.x] = before + incl - mine;
+      __syncthreads();
+      for (int i = threadIdx.x; i - lane < total; i += kHubThreads) {
+        const bool has = i < total;
+        int lo = 0, hi = nk - 1;  // the last run starting at or before i
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (sh->hist[mid] <= i) lo = mid; else hi = mid - 1;
+        }
+        const int64_t at = out0 + sh->base[lo] + (i - sh->hist[lo]);
+        const int32_t c = has ? __ldcg(&h.out_c[at]) : -1;
+        const double w = has ? __ldcg(&h.out_w[at]) : 0.0;
         bool fresh = false;
         uint32_t s = hash_slot(c, mask);
-        if (mine && *(volatile int *)&sh->over == 0) {
+        if (has && ((mix32((uint32_t)c) >> 12) & smask) == share &&
+            *(volatile int *)&sh->over == 0) {
           while (true) {
-            int32_t x = keys[s];
-            if (x == -1) {
-              x = atomicCAS(&keys[s], -1, c);
-              fresh = x == -1;
-            }
+            const int32_t x = atomicCAS(&keys[s], -1, c);
+            fresh = x == -1;
             if (x == -1 || x == c) break;
             s = (s + 1) & mask;
           }
@@ -97,17 +130,17 @@ __device__ __forceinline__ void hub_merge(const SweepArgs &a, const HubWork &h, 
         }
         const unsigned fm = __ballot_sync(FULL, fresh);
         if (fm) {
-          int at = 0;
-          if (lane == 0) at = atomicAdd(&sh->count, __popc(fm));
-          at = __shfl_sync(FULL, at, 0) + __popc(fm & ((1u << lane) - 1u));
+          int n = 0;
+          if (lane == 0) n = atomicAdd(&sh->count, __popc(fm));
+          n = __shfl_sync(FULL, n, 0) + __popc(fm & ((1u << lane) - 1u));
           if (fresh) {
-            if (at < kHubList) list[at] = (uint16_t)s;
+            if (n < kHubList) list[n] = (uint16_t)s;
             else sh->over = 1;
           }
         }
       }
+      __syncthreads();  // the pairs are in the table, the runs' offsets read
     }
-    __syncthreads();
     if (sh->over) {  // block-uniform: start over with twice the shares
       __syncthreads();
       for (int q = threadIdx.x; q < kHubTableCap; q += kHubThreads) {

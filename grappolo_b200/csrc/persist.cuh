@@ -285,45 +285,52 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_sweep_iteration(IterArgs
                         tkeys, tvals, &s_cluster, s_g, s_c);
       GLV_QTRACE(s, 3, threadIdx.x == 0);
     }
-    if (t_hub + t_blk + t_seg > 0) {
-      // hub chunks, then block rows, then hub partitions (which wait for
+    // The rows of 128..1023 entries of a step with few of them (at most
+    // gridDim / 4, and no more than the blocks left) go to whole blocks: 1 or 2
+    // rounds instead of up to 8.  With more, four rows per block are better:
+    // R-MAT 20, whose steps hold 50 to 800, took 3% longer with as many on
+    // blocks as the grid could take, while steps of a row or two (the last
+    // levels of a planted partition) go from 12.3 to 9.5 us.
+    const int nteam = st.seg[BIN_T256 + 1] - st.seg[BIN_T128];
+    const int n_up = (4 * nteam <= (int)gridDim.x &&
+                      nteam + t_hub + t_blk + t_seg <= (int)gridDim.x) ? nteam : 0;
+    if (t_hub + t_blk + n_up + t_seg > 0) {
+      // hub chunks, block rows, team rows, then hub partitions (which wait for
       // their hub's chunks: every chunk is handed out before any partition)
       unsigned *ctr = &p.task_ctr[3 * s];
       if (thread_id() == 0) s_task[0] = (int)atomicAdd(ctr, 1u);
       __syncthreads();
       for (unsigned it = 0;; ++it) {
         int t = s_task[it & 1];
-        if (t >= st.hub_chunk[1] - st.hub_chunk[0] + st.seg[BIN_BLOCK + 1] - st.seg[BIN_BLOCK] +
-                     st.hub_segs[1] - st.hub_segs[0])
-          break;
+        if (t >= t_hub + t_blk + n_up + t_seg) break;
         const int nxt = (thread_id() == 0) ? (int)atomicAdd(&p.task_ctr[3 * s], 1u) : 0;
-        if (t < st.hub_chunk[1] - st.hub_chunk[0]) {
+        if (t < t_hub) {
           hub_chunk_task(p.a, p.h, st.hub_chunk[0] + t, tkeys, tvals, fill, &s_hub, s_g, s_c);
+        } else if ((t -= t_hub) < t_blk + n_up) {
+          const int n256 = st.seg[BIN_T256 + 1] - st.seg[BIN_T256];
+          int pos = st.seg[BIN_BLOCK] + t;
+          if ((t -= t_blk) >= 0)
+            pos = (t < n256) ? st.seg[BIN_T256] + t : st.seg[BIN_T128] + (t - n256);
+          row_vertex<512>(p.a, pos, tkeys, tvals, fill, 0, s_self, s_own, s_g, s_c);
         } else {
-          t -= st.hub_chunk[1] - st.hub_chunk[0];
-          const int nblk = st.seg[BIN_BLOCK + 1] - st.seg[BIN_BLOCK];
-          if (t < nblk)
-            row_vertex<512>(p.a, st.seg[BIN_BLOCK] + t, tkeys, tvals, fill, 0, s_self, s_own, s_g,
-                            s_c);
-          else
-            hub_part_task(p.a, p.h, st.hub_segs[0] + (t - nblk), tkeys, tvals, fill, &s_hub, s_g,
-                          s_c);
+          hub_part_task(p.a, p.h, st.hub_segs[0] + (t - t_blk - n_up), tkeys, tvals, fill, &s_hub,
+                        s_g, s_c);
         }
         if (thread_id() == 0) s_task[(it + 1) & 1] = nxt;
         __syncthreads();
       }
       GLV_QTRACE(s, 0, threadIdx.x == 0);
     }
-    if (st.seg[BIN_T256 + 1] > st.seg[BIN_T128]) {
+    if (nteam > n_up) {
       const int team = thread_id() / kTeamThreads, tt = thread_id() % kTeamThreads;
-      if (tt == 0) s_team_task[team][0] = (int)atomicAdd(&p.task_ctr[3 * s + 1], 1u);
+      if (tt == 0) s_team_task[team][0] = n_up + (int)atomicAdd(&p.task_ctr[3 * s + 1], 1u);
       team_sync<128>(team);
       for (unsigned it = 0;; ++it) {
         const int t = s_team_task[team][it & 1];
         // the longer rows (the T256 bin, after the T128 bin in member order) first
         const int n256 = st.seg[BIN_T256 + 1] - st.seg[BIN_T256];
-        if (t >= st.seg[BIN_T256 + 1] - st.seg[BIN_T128]) break;
-        const int nxt = (tt == 0) ? (int)atomicAdd(&p.task_ctr[3 * s + 1], 1u) : 0;
+        if (t >= nteam) break;
+        const int nxt = (tt == 0) ? n_up + (int)atomicAdd(&p.task_ctr[3 * s + 1], 1u) : 0;
         const int pos = (t < n256) ? st.seg[BIN_T256] + t : st.seg[BIN_T128] + (t - n256);
         row_vertex<128>(p.a, pos, tkeys + team * kTeamCap, tvals + team * kTeamCap,
                         fill + team * (kPersistFill * kTeamThreads / kPersistThreads), team,
