@@ -14,7 +14,7 @@
 // made a round as long as its longest row: R-MAT 20, whose rows on that chain
 // sum to 5.8 M entries, took 182 ms, R-MAT 22 (edge factor 14) 583 ms, the
 // 100k partition 10.6 ms.  Here nothing waits for a round; the same colourings
-// take 15.7, 31.7 and 5.2 ms:
+// take 7.5, 13.9 and 3.7 ms:
 //
 // * one 64-bit word per vertex holds the higher-priority neighbours not yet
 //   coloured (high half) and the colours 0..31 they took (low half).  A vertex
@@ -42,9 +42,14 @@
 namespace glv {
 
 constexpr int kFlowThreads = 256;
-constexpr int kFlowUnroll = 4;                          // entries a lane has in flight
+// Blocks per SM of the dataflow kernel.  Idle warps poll, and polling slows the
+// atomics of the others: 4 blocks took 17.3 ms on R-MAT 20's second level, 2 or 1
+// 12.0; a batch of 200 graphs, with work for every warp, 18.4 ms with 2 and
+// 22.1 with 1.
+constexpr int kFlowBlocks = 2;
 constexpr int kFlowChunk = 512;                         // fewest entries of a split row's task
 constexpr int64_t kFlowMaxParts = (int64_t)1 << 20;     // tasks of one row (21 bits of a task word)
+constexpr int kFlowCtr = 16;                            // counters on lines of their own (128 B)
 constexpr int kFlowChain = 64;                          // own next vertices before one is published
 constexpr unsigned long long kFlowEmpty = ~0ull;
 constexpr unsigned long long kFlowStallNs = 5000000000ull;
@@ -61,7 +66,7 @@ struct ColorFlow {
   int32_t *color;
   unsigned long long *queue;  // task words (kFlowEmpty = not yet published)
   unsigned long long qcap;
-  unsigned long long *ctr;    // {next ticket, tasks published, tasks finished}
+  unsigned long long *ctr;    // next ticket, tasks published, tasks finished, kFlowCtr apart
   int32_t *status;            // [0] a vertex needs more than kMaxColors, [1] no progress
 };
 
@@ -171,7 +176,7 @@ __device__ __forceinline__ void flow_publish(const ColorFlow &f, int32_t v, int3
   const int total = __shfl_sync(FULL, incl, 31);
   if (total == 0) return;
   unsigned long long base = 0;
-  if (lane == 0) base = atomicAdd(&f.ctr[1], (unsigned long long)total);
+  if (lane == 0) base = atomicAdd(&f.ctr[kFlowCtr], (unsigned long long)total);
   base = __shfl_sync(FULL, base, 0) + (unsigned long long)(incl - mine);
   for (int64_t p = 0; p < mine; ++p)
     if (base + p < f.qcap)
@@ -219,31 +224,34 @@ __global__ void __launch_bounds__(kFlowThreads) k_color_flow(ColorFlow f) {
     if (lane == 0) {
       const unsigned long long t = atomicAdd(&f.ctr[0], 1ull);
       unsigned long long seen = 0, since = 0;
+      unsigned pause = 20;
       for (unsigned it = 0;; ++it) {
         if (t < f.qcap) {
           task = *(volatile unsigned long long *)&f.queue[t];
           if (task != kFlowEmpty) break;
         }
-        if ((it & 7u) == 0) {
+        if ((it & 15u) == 15u) {
           // finished first: it never passes the published count, so equal
           // values mean that no task is running or waiting
-          const unsigned long long fin = *(volatile unsigned long long *)&f.ctr[2];
+          const unsigned long long fin = *(volatile unsigned long long *)&f.ctr[2 * kFlowCtr];
           __threadfence();
-          const unsigned long long pub = *(volatile unsigned long long *)&f.ctr[1];
+          const unsigned long long pub = *(volatile unsigned long long *)&f.ctr[kFlowCtr];
           if (fin == pub) break;
-          if ((it & 1023u) == 0) {
-            unsigned long long now;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-            if (since == 0 || fin + pub != seen) {
-              seen = fin + pub;
-              since = now;
-            } else if (now - since > kFlowStallNs) {
-              atomicExch(&f.status[1], 1);
-              break;
-            }
+          unsigned long long now;
+          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+          if (since == 0 || fin + pub != seen) {
+            seen = fin + pub;
+            since = now;
+          } else if (now - since > kFlowStallNs) {
+            atomicExch(&f.status[1], 1);
+            break;
           }
+          // Tasks come in ticket order: the warps next in line poll, the
+          // others sleep longer the more tickets are before theirs.
+          const unsigned long long ahead = t >= pub ? t - pub : 0;
+          pause = ahead < 16 ? 20u : (ahead < 512 ? 20u + (unsigned)ahead : 512u);
         }
-        __nanosleep(it < 16 ? 20 : 100);
+        __nanosleep(pause);
       }
     }
     task = __shfl_sync(FULL, task, 0);
@@ -257,78 +265,55 @@ __global__ void __launch_bounds__(kFlowThreads) k_color_flow(ColorFlow f) {
       const unsigned long long bit = 1ull << (c & 31);
       int32_t nv_ = -1, nc = 0;  // the ready vertex this warp keeps
       int64_t nrb = 0, ndeg = 0, ns0 = 0;
-      for (int64_t base = jb; base < je; base += 32 * kFlowUnroll) {
-        int32_t u[kFlowUnroll];
-        bool low[kFlowUnroll];
-        unsigned long long old[kFlowUnroll];
-#pragma unroll
-        for (int q = 0; q < kFlowUnroll; ++q) {
-          const int64_t j = base + 32 * q + lane;
-          u[q] = (j < je) ? f.tail[j] : v;
-        }
-#pragma unroll
-        for (int q = 0; q < kFlowUnroll; ++q)
-          low[q] = u[q] != v && prio_before(v, u[q], f.hashed, f.seed);
+      for (int64_t base = jb; base < je; base += 32) {
+        const int32_t u = (base + lane < je) ? f.tail[base + lane] : v;
+        const bool low = u != v && prio_before(v, u, f.hashed, f.seed);
         if (c < 32) {
-#pragma unroll
-          for (int q = 0; q < kFlowUnroll; ++q)
-            if (low[q]) atomicOr(&f.word[u[q]], bit);
+          if (low) atomicOr(&f.word[u], bit);
         } else {
-#pragma unroll
-          for (int q = 0; q < kFlowUnroll; ++q) {
-            if (!low[q]) continue;
-            const int64_t p0 = f.ptr[u[q]], p1 = f.ptr[u[q] + 1];
+          if (low) {
+            const int64_t p0 = f.ptr[u], p1 = f.ptr[u + 1];
             if ((c >> 5) < (p1 - p0 + 32) / 32)  // colours past the degree never block u
-              atomicOr(&f.ext[flow_ext_base(p0, u[q]) + (c >> 5)], (uint32_t)bit);
+              atomicOr(&f.ext[flow_ext_base(p0, u) + (c >> 5)], (uint32_t)bit);
           }
           __threadfence();
         }
-        bool any = false;
-#pragma unroll
-        for (int q = 0; q < kFlowUnroll; ++q) {
-          old[q] = low[q] ? atomicAdd(&f.word[u[q]], 0xFFFFFFFF00000000ull) : 0ull;
-          any = any || (old[q] >> 32) == 1ull;
+        const unsigned long long old = low ? atomicAdd(&f.word[u], 0xFFFFFFFF00000000ull) : 0ull;
+        const bool ready = (old >> 32) == 1ull;
+        if (!__any_sync(FULL, ready)) continue;
+        const int64_t p0 = ready ? f.ptr[u] : 0;
+        const int64_t dg = ready ? f.ptr[u + 1] - p0 : 0;
+        const int32_t st = ready ? f.start[u] : 0;
+        const uint32_t fr = ~(uint32_t)old;
+        int cu = fr ? __ffs(fr) - 1 : 0;
+        unsigned full = __ballot_sync(FULL, ready && fr == 0);
+        if (full) __threadfence();  // the bitmap words ordered before the count
+        while (full) {  // warp-uniform
+          const int src = __ffs(full) - 1;
+          full &= full - 1;
+          const int x = flow_first_free(f, __shfl_sync(FULL, u, src), __shfl_sync(FULL, p0, src),
+                                        __shfl_sync(FULL, dg, src));
+          if (lane == src) cu = x;
         }
-        if (!__any_sync(FULL, any)) continue;
-        const bool last = base + 32 * kFlowUnroll >= je && chain < kFlowChain;
-#pragma unroll
-        for (int q = 0; q < kFlowUnroll; ++q) {
-          const bool ready = (old[q] >> 32) == 1ull;
-          const unsigned rm = __ballot_sync(FULL, ready);
-          if (rm == 0) continue;
-          const int64_t p0 = ready ? f.ptr[u[q]] : 0;
-          const int64_t dg = ready ? f.ptr[u[q] + 1] - p0 : 0;
-          const int32_t st = ready ? f.start[u[q]] : 0;
-          const uint32_t fr = ~(uint32_t)old[q];
-          int cu = fr ? __ffs(fr) - 1 : 0;
-          unsigned full = __ballot_sync(FULL, ready && fr == 0);
-          if (full) __threadfence();  // the bitmap words ordered before the count
-          while (full) {  // warp-uniform
-            const int src = __ffs(full) - 1;
-            full &= full - 1;
-            const int x = flow_first_free(f, __shfl_sync(FULL, u[q], src),
-                                          __shfl_sync(FULL, p0, src), __shfl_sync(FULL, dg, src));
-            if (lane == src) cu = x;
-          }
-          if (cu >= kMaxColors) {
-            atomicExch(&f.status[0], 1);
-            cu = kMaxColors - 1;
-          }
-          if (ready) f.color[u[q]] = cu;
-          const int64_t n = (ready && dg > st) ? flow_parts(dg - st) : 0;
-          const unsigned pm = __ballot_sync(FULL, n > 0);
-          int64_t first = 0;
-          if (last && nv_ < 0 && pm) {  // keep the first ready vertex with a row to send
-            const int src = __ffs(pm) - 1;
-            nv_ = __shfl_sync(FULL, u[q], src);
-            nc = __shfl_sync(FULL, cu, src);
-            nrb = __shfl_sync(FULL, p0, src);
-            ndeg = __shfl_sync(FULL, dg, src);
-            ns0 = __shfl_sync(FULL, st, src);
-            if (lane == src) first = 1;
-          }
-          flow_publish(f, u[q], cu, first, n);
+        if (cu >= kMaxColors) {
+          atomicExch(&f.status[0], 1);
+          cu = kMaxColors - 1;
         }
+        if (ready) f.color[u] = cu;
+        const int64_t n = (ready && dg > st) ? flow_parts(dg - st) : 0;
+        const unsigned pm = __ballot_sync(FULL, n > 0);
+        int64_t first = 0;
+        if (base + 32 >= je && chain < kFlowChain && pm) {
+          // keep the first ready vertex with a row to send
+          const int src = __ffs(pm) - 1;
+          nv_ = __shfl_sync(FULL, u, src);
+          nc = __shfl_sync(FULL, cu, src);
+          nrb = __shfl_sync(FULL, p0, src);
+          ndeg = __shfl_sync(FULL, dg, src);
+          ns0 = __shfl_sync(FULL, st, src);
+          if (lane == src) first = 1;
+        }
+        flow_publish(f, u, cu, first, n);
       }
       if (nv_ < 0) break;
       v = nv_; c = nc; part = 0;
@@ -337,7 +322,7 @@ __global__ void __launch_bounds__(kFlowThreads) k_color_flow(ColorFlow f) {
     __syncwarp();
     if (lane == 0) {
       __threadfence();  // this task's publications before its end
-      atomicAdd(&f.ctr[2], 1ull);
+      atomicAdd(&f.ctr[2 * kFlowCtr], 1ull);
     }
   }
 }

@@ -871,13 +871,13 @@ int Engine::color_jp(const Level &L, int *ncolors) {
   f.qcap = (unsigned long long)(L.nv + L.nnz / kFlowChunk + 1);
   int32_t *maxc;
   TRY(alloc(&f.word, L.nv)); TRY(alloc(&f.start, L.nv)); TRY(alloc(&f.ext, next));
-  TRY(alloc(&f.queue, f.qcap)); TRY(alloc(&f.ctr, 3)); TRY(alloc(&f.status, 2));
+  TRY(alloc(&f.queue, f.qcap)); TRY(alloc(&f.ctr, 3 * kFlowCtr)); TRY(alloc(&f.status, 2));
   TRY(alloc(&maxc, 1));
   CK(cudaMemsetAsync(f.word, 0, L.nv * sizeof(unsigned long long), s_));
   CK(cudaMemsetAsync(f.start, 0x7f, L.nv * sizeof(int32_t), s_));
   CK(cudaMemsetAsync(f.ext, 0, next * sizeof(uint32_t), s_));
   CK(cudaMemsetAsync(f.queue, 0xff, f.qcap * sizeof(unsigned long long), s_));
-  CK(cudaMemsetAsync(f.ctr, 0, 3 * sizeof(unsigned long long), s_));
+  CK(cudaMemsetAsync(f.ctr, 0, 3 * kFlowCtr * sizeof(unsigned long long), s_));
   CK(cudaMemsetAsync(f.status, 0, 2 * sizeof(int32_t), s_));
   CK(cudaMemsetAsync(maxc, 0xff, sizeof(int32_t), s_));
   if (L.nnz > 0) {
@@ -888,7 +888,7 @@ int Engine::color_jp(const Level &L, int *ncolors) {
   }
   LAUNCH(k_flow_seed, grid_for(L.nv, 256, nsm_ * 8), 256, 0, s_, f);
   if (L.nnz > 0)
-    LAUNCH(k_color_flow, grid_for(L.nv, 32, nsm_ * 4), kFlowThreads, 0, s_, f);
+    LAUNCH(k_color_flow, grid_for(L.nv, 32, nsm_ * kFlowBlocks), kFlowThreads, 0, s_, f);
   LAUNCH(k_max_color, grid_for(L.nv, 256, nsm_ * 8), 256, 0, s_, L.nv, color_, maxc);
   int32_t h[2], hm;
   CK(cudaMemcpyAsync(h, f.status, sizeof(h), cudaMemcpyDeviceToHost, s_));
