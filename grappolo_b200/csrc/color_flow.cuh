@@ -93,7 +93,7 @@ __device__ __forceinline__ unsigned long long flow_task(int32_t v, int32_t c, in
 struct FlowTileSmem {
   int32_t cnt[kMergeTile + 1];
   int32_t first[kMergeTile + 1];
-  int32_t off[kMergeTile + 2];
+  TileRows rows;
 };
 
 __global__ void __launch_bounds__(kFlowThreads) k_flow_counts(ColorFlow f, int64_t nnz,
@@ -111,24 +111,18 @@ __global__ void __launch_bounds__(kFlowThreads) k_flow_counts(ColorFlow f, int64
     if (j1 <= j0) continue;  // only row ends (tile-uniform)
     const int64_t ih = min(i1, nv - 1);
     const int nr = (int)(ih - i0 + 1);
-    for (int k = threadIdx.x; k <= nr; k += kFlowThreads) {
-      const int64_t r = f.ptr[i0 + k] - j0;
-      sm.off[k] = (int32_t)max((int64_t)0, min(r, (int64_t)kMergeTile + 1));
-      if (k < nr) { sm.cnt[k] = 0; sm.first[k] = INT32_MAX; }
-    }
-    __syncthreads();
     const int ne = (int)(j1 - j0);
+    for (int k = threadIdx.x; k < nr; k += kFlowThreads) {
+      sm.cnt[k] = 0;
+      sm.first[k] = INT32_MAX;
+    }
+    tile_rows_fill(&sm.rows, f.ptr, i0, nr, j0, ne);
     for (int q0 = 0; q0 < ne; q0 += kFlowThreads) {  // ne is the tile's: warp-uniform
       const int q = q0 + (int)threadIdx.x;
       const bool has = q < ne;
-      int lo = 0;
+      const int lo = tile_row(&sm.rows, q, ne);
       bool before = false, after = false;
       if (has) {
-        int hi = nr - 1;  // the last row starting at or before q
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (sm.off[mid] <= q) lo = mid; else hi = mid - 1;
-        }
         const int32_t v = (int32_t)(i0 + lo), u = f.tail[j0 + q];
         if (u != v) {
           before = prio_before(u, v, f.hashed, f.seed);

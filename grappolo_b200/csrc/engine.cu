@@ -633,9 +633,9 @@ int Engine::init(int64_t nv0, int64_t nnz0) {
     if (v >= 1 && (v & (v - 1)) == 0) cluster_parts_ = v;
   }
   TRY(alloc(&cst, 4));
-  // partials of the modularity pass (one per 256 vertices) and of the
-  // constant's reduction (kConstParts blocks) share these buffers
-  const size_t nparts = std::max<size_t>((n + kModVB - 1) / kModVB, kConstParts) + 1;
+  // partials of the modularity pass (one per block) and of the constant's
+  // reduction (kConstParts blocks) share these buffers
+  const size_t nparts = kConstParts + 1;
   TRY(alloc(&part_e_, nparts)); TRY(alloc(&part_a_, nparts)); TRY(alloc(&mod_out_, 8));
   CK(cudaMallocHost((void **)&h_mod_, 8 * sizeof(double)));
   CK(cudaMemsetAsync(dDeg, 0, n * sizeof(double), s_));
@@ -4063,7 +4063,8 @@ namespace glv {
 // vertices, 65,536 pairs -> 16,777,216 vertices, 1 MiB of device memory that
 // every GPU which loads this library keeps until the process exits.
 constexpr int64_t kStaticModParts = 65536;
-constexpr int64_t kStaticModMaxVertices = kStaticModParts * kModVB;
+constexpr int64_t kStaticModMaxVertices = 16777216;  // the documented limit of the entry
+constexpr int64_t kStaticModBlocks = 148 * 4;
 
 // Block partials of e_xx (first half) and a2_x (second half).  Shared by every
 // call on a device: concurrent calls on that device race on it.
@@ -4071,6 +4072,77 @@ static __device__ __align__(256) double g_mod_scratch[2 * kStaticModParts];
 
 static std::mutex g_mod_scratch_mu;
 static double *g_mod_scratch_addr[kMaxDevices];  // device address of g_mod_scratch, per device
+
+// Rows ended before item d of the merge sequence: the largest i in [lo, hi]
+// with ptr[i] + i <= d (strictly increasing; lo satisfies it).  All threads of
+// the block search together, one 257th of the range per round; s_hit is block
+// scratch.  Ends with a barrier.
+__device__ __forceinline__ int64_t block_split(const int64_t *ptr, int64_t d, int64_t lo,
+                                               int64_t hi, int *s_hit) {
+  while (lo < hi) {
+    const int64_t step = (hi - lo + blockDim.x - 1) / blockDim.x;  // >= 1
+    if (threadIdx.x == 0) *s_hit = 0;
+    __syncthreads();
+    const int64_t i = lo + step * (threadIdx.x + 1);
+    if (i <= hi && ptr[i] + i <= d) atomicMax(s_hit, (int)threadIdx.x + 1);
+    __syncthreads();
+    const int h = *s_hit;
+    __syncthreads();
+    lo += step * h;
+    hi = min(hi, lo + step - 1);
+  }
+  return lo;
+}
+
+// Block partials of e_xx and a2_x over merge-path tiles (modularity_merge_tile
+// without a split array: every block takes a run of tiles, searches its first
+// row, and finds a tile's last row while it has the rows at hand).  A vertex
+// labelled -1 belongs to no community: its entries add nothing.  Blocks of 256
+// vertices each took 6.65 ms on R-MAT 22 (123M entries), as long as the block
+// that holds the hubs; equal tiles take 0.91 ms
+// (12 B per entry and 16 B per vertex: 1.5 GB, 0.24 ms at the measured copy rate;
+// the 123M gathers of C move 3.9 GB of L2 sectors).
+__global__ void __launch_bounds__(256) k_modularity_static(int64_t nv, const int64_t *ptr,
+                                                           const int32_t *tail, const double *w,
+                                                           const int32_t *C, const double *cDeg,
+                                                           double *part_e, double *part_a) {
+  __shared__ MergeSmem sm;
+  __shared__ double sh[8];
+  __shared__ int s_hit;
+  const int64_t nnz = ptr[nv], ntiles = merge_tiles(nv, nnz);
+  const int64_t tb = ntiles * blockIdx.x / gridDim.x, te = ntiles * (blockIdx.x + 1) / gridDim.x;
+  double ex = 0.0, a2 = 0.0;
+  int64_t i0 = 0;
+  if (te > tb) {
+    const int64_t d = tb * (int64_t)kMergeTile;
+    i0 = block_split(ptr, d, max((int64_t)0, d - nnz), min(d, nv), &s_hit);
+  }
+  for (int64_t tile = tb; tile < te; ++tile) {
+    const int64_t d0 = tile * (int64_t)kMergeTile;
+    const int64_t d1 = min(d0 + (int64_t)kMergeTile, nv + nnz);
+    const int64_t i1 =
+        block_split(ptr, d1, max(i0, d1 - nnz), min(i0 + (d1 - d0), nv), &s_hit);
+    const int64_t j0 = d0 - i0, j1 = d1 - i1;
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += 256) {
+      const double dg = cDeg[i];
+      a2 = __dadd_rn(a2, __dmul_rn(dg, dg));
+    }
+    if (j1 > j0) {  // block-uniform
+      const int nr = (int)(min(i1, nv - 1) - i0 + 1), ne = (int)(j1 - j0);
+      for (int k = threadIdx.x; k < nr; k += 256) {
+        const int32_t c = C[i0 + k];
+        sm.comm[k] = c >= 0 ? c : INT32_MIN;
+      }
+      tile_rows_fill(&sm.rows, ptr, i0, nr, j0, ne);
+      modularity_entries<256, 8>(j0, ne, tail, w, C, &sm, ex);
+    }
+    i0 = i1;
+    __syncthreads();
+  }
+  ex = block_sum<256>(ex, sh);
+  a2 = block_sum<256>(a2, sh);
+  if (threadIdx.x == 0) { part_e[blockIdx.x] = ex; part_a[blockIdx.x] = a2; }
+}
 
 // The fold of k_modularity_final with the constant passed by value, so the
 // call needs no device copy of it.
@@ -4131,12 +4203,13 @@ extern "C" int glv_dev_modularity_static(long nv, const long *d_ptr, const int *
     scratch = g_mod_scratch_addr[dev];
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int nparts = (int)((nv + kModVB - 1) / kModVB);
+  // four blocks per SM, fewer where the vertices do not give each 32 rows
+  const int nparts = (int)std::max<int64_t>(8, std::min<int64_t>(nv / 32, kStaticModBlocks));
   double *part_e = scratch, *part_a = scratch + kStaticModParts;
-  // Every partial read below is written first by this call's k_modularity_part,
-  // so nothing in the scratch needs clearing.
-  k_modularity_part<<<nparts, 256, 0, s>>>(nv, (const int64_t *)d_ptr, d_tail, d_weight, d_C,
-                                           nullptr, d_cDeg, part_e, part_a);
+  // Every partial read below is written first by this call's
+  // k_modularity_static, so nothing in the scratch needs clearing.
+  k_modularity_static<<<nparts, 256, 0, s>>>(nv, (const int64_t *)d_ptr, d_tail, d_weight, d_C,
+                                             d_cDeg, part_e, part_a);
   k_modularity_final_value<<<1, 256, 0, s>>>(nparts, part_e, part_a, constant, d_out);
   g_launches += 2;
   CK(cudaGetLastError());

@@ -101,45 +101,6 @@ __global__ void k_constant_from_partials(int nparts, const double *part, double 
 //  BasicCommunitiesDetection/parallelLouvainMethod.cpp:247-255).
 // Colour phases compute cWI[i] = sum_{j: C[tail]==C[i]} w here; Jacobi phases
 // pass the per-vertex Counter[own] their sweep produced (own_w).
-// Each block takes 256 consecutive vertices and walks their edges
-// edge-parallel, so hub rows do not serialise one lane.
-constexpr int kModVB = 256;
-
-__global__ void __launch_bounds__(256) k_modularity_part(int64_t nv, const int64_t *ptr,
-                                                         const int32_t *tail, const double *w,
-                                                         const int32_t *C, const double *own_w,
-                                                         const double *cDeg, double *part_e,
-                                                         double *part_a) {
-  __shared__ int64_t s_ptr[kModVB + 1];
-  __shared__ int32_t s_c[kModVB];
-  __shared__ double sh[8];
-  const int64_t v0 = (int64_t)blockIdx.x * kModVB;
-  const int64_t v1 = min(nv, v0 + kModVB);
-  const int nvb = (int)(v1 - v0);
-  double a2 = 0.0, ex = 0.0;
-  if (threadIdx.x < nvb) {
-    const double d = cDeg[v0 + threadIdx.x];
-    a2 = __dmul_rn(d, d);
-  }
-  if (own_w) {
-    if (threadIdx.x < nvb) ex = own_w[v0 + threadIdx.x];
-  } else {
-    for (int k = threadIdx.x; k <= nvb; k += blockDim.x) s_ptr[k] = ptr[v0 + k];
-    for (int k = threadIdx.x; k < nvb; k += blockDim.x) s_c[k] = C[v0 + k];
-    __syncthreads();
-    const int64_t eb = s_ptr[0], ee = s_ptr[nvb];
-    int h = 0;
-    for (int64_t e = eb + threadIdx.x; e < ee; e += blockDim.x) {
-      while (s_ptr[h + 1] <= e) ++h;
-      // a vertex labelled -1 belongs to no community: its entries add nothing
-      if (s_c[h] >= 0 && C[tail[e]] == s_c[h]) ex = __dadd_rn(ex, w[e]);
-    }
-  }
-  ex = block_sum<256>(ex, sh);
-  a2 = block_sum<256>(a2, sh);
-  if (threadIdx.x == 0) { part_e[blockIdx.x] = ex; part_a[blockIdx.x] = a2; }
-}
-
 // Merge-path tiles.  The items of a level are its rows' entries interleaved
 // with one "row end" per row (row i's entries come before its end), nv + nnz
 // items in all; a tile is kMergeTile consecutive items.  A hub row is cut over
@@ -167,10 +128,58 @@ __global__ void k_merge_splits(int64_t nv, int64_t nnz, const int64_t *ptr, int6
   }
 }
 
-// Shared memory of one merge tile: row starts relative to the tile's first
-// entry (clamped to [0, kMergeTile + 1]) and the rows' communities.
+// The rows of one tile's entries in shared memory.  Entry q (of the ne <=
+// kMergeTile entries from j0 on) belongs to the last row starting at or before
+// it: a row marks the entry it starts at, a warp takes the last mark among the
+// entries up to its lane's, and the row of each 32nd entry is searched once.
+// (A binary search of 12 shared loads for every entry made the modularity pass
+// of 110M entries 1.4 ms; with the marks 1.0.)
+struct TileRows {
+  int32_t off[kMergeTile + 2];       // row starts relative to j0, clamped to [0, kMergeTile + 1]
+  int16_t start[kMergeTile];         // row starting at an entry, or -1
+  int16_t first[kMergeTile / 32];    // row of every 32nd entry
+};
+static_assert(kMergeTile < 32767 && kMergeTile % 64 == 0, "16-bit row numbers, whole words");
+
+// Fills tr for rows i0 .. i0 + nr - 1; all threads of the block call.  Ends
+// with a barrier; the caller puts one between the last use and the next fill.
+__device__ __forceinline__ void tile_rows_fill(TileRows *tr, const int64_t *ptr, int64_t i0, int nr,
+                                               int64_t j0, int ne) {
+  for (int k = threadIdx.x; k <= nr; k += blockDim.x) {
+    const int64_t r = ptr[i0 + k] - j0;
+    tr->off[k] = (int32_t)max((int64_t)0, min(r, (int64_t)kMergeTile + 1));
+  }
+  for (int k = threadIdx.x; 2 * k < ne; k += blockDim.x)
+    reinterpret_cast<int32_t *>(tr->start)[k] = -1;
+  __syncthreads();
+  for (int k = threadIdx.x; k < nr; k += blockDim.x) {
+    const int o = tr->off[k];
+    if (o < ne && tr->off[k + 1] > o) tr->start[o] = (int16_t)k;
+  }
+  for (int g = threadIdx.x; 32 * g < ne; g += blockDim.x) {
+    int lo = 0, hi = nr - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (tr->off[mid] <= 32 * g) lo = mid; else hi = mid - 1;
+    }
+    tr->first[g] = (int16_t)lo;
+  }
+  __syncthreads();
+}
+
+// Row of entry q (relative to i0); every lane of the warp calls, with q - lane a
+// multiple of 32.  Lanes with q >= ne get a row that means nothing.
+__device__ __forceinline__ int tile_row(const TileRows *tr, int q, int ne) {
+  const int lane = threadIdx.x & 31;
+  const int s = (q < ne) ? tr->start[q] : -1;
+  const unsigned m = __ballot_sync(FULL, s >= 0) & (0xffffffffu >> (31 - lane));
+  const int r = __shfl_sync(FULL, s, m ? 31 - __clz(m) : 0);
+  return m ? r : (q - lane < ne ? tr->first[q >> 5] : 0);
+}
+
+// Shared memory of one merge tile: its rows and their communities.
 struct MergeSmem {
-  int32_t off[kMergeTile + 2];
+  TileRows rows;
   int32_t comm[kMergeTile + 1];
 };
 
@@ -184,7 +193,7 @@ struct MergeSmem {
 constexpr int kRowSumThreads = 256;
 struct RowSumSmem {
   double acc[kMergeTile + 1];
-  int32_t off[kMergeTile + 2];
+  TileRows rows;
 };
 
 __global__ void __launch_bounds__(kRowSumThreads) k_row_sums_tiles(int64_t nv, int64_t nnz,
@@ -205,26 +214,14 @@ __global__ void __launch_bounds__(kRowSumThreads) k_row_sums_tiles(int64_t nv, i
     // rows holding entries j0..j1-1: i0 .. ih
     const int64_t ih = min(i1, nv - 1);
     const int nr = (int)(ih - i0 + 1);
-    for (int k = threadIdx.x; k <= nr; k += kRowSumThreads) {
-      const int64_t r = ptr[i0 + k] - j0;
-      sm.off[k] = (int32_t)max((int64_t)0, min(r, (int64_t)kMergeTile + 1));
-      if (k < nr) sm.acc[k] = 0.0;
-    }
-    __syncthreads();
     const int ne = (int)(j1 - j0);
+    for (int k = threadIdx.x; k < nr; k += kRowSumThreads) sm.acc[k] = 0.0;
+    tile_rows_fill(&sm.rows, ptr, i0, nr, j0, ne);
     for (int q0 = 0; q0 < ne; q0 += kRowSumThreads) {  // ne is the tile's: warp-uniform
       const int q = q0 + (int)threadIdx.x;
       const bool has = q < ne;
-      int lo = 0;
-      double x = 0.0;
-      if (has) {
-        int hi = nr - 1;  // the last row starting at or before q
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (sm.off[mid] <= q) lo = mid; else hi = mid - 1;
-        }
-        x = w[j0 + q];
-      }
+      const int lo = tile_row(&sm.rows, q, ne);
+      double x = has ? w[j0 + q] : 0.0;
       // the warp's entries come in row order: a segmented inclusive scan
       // leaves each row's warp sum in its last lane
       const int key = has ? lo : -1 - lane;
@@ -260,6 +257,35 @@ __global__ void k_init_phase_fill(int64_t nv, const double *vDeg, double *cDeg, 
   }
 }
 
+// Adds the weights of a tile's entries whose two ends share a community to ex.
+// U entries per thread are in flight: 8 where the registers allow it (the
+// gathers of C bound the pass; 4 took 1.35 ms on R-MAT 22's 123M entries, 8
+// 0.91), 4 in the persistent sweep's 64.
+template <int NT, int U>
+__device__ __forceinline__ void modularity_entries(int64_t j0, int ne, const int32_t *tail,
+                                                   const double *w, const int32_t *C,
+                                                   const MergeSmem *sm, double &ex) {
+  for (int q0 = 0; q0 < ne; q0 += U * NT) {  // block-uniform
+    int32_t t[U], c[U];
+    double x[U];
+    int row[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = q0 + u * NT + (int)threadIdx.x;
+      t[u] = (q < ne) ? __ldcs(&tail[j0 + q]) : -1;
+      x[u] = (q < ne) ? __ldcs(&w[j0 + q]) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) c[u] = (t[u] >= 0) ? C[t[u]] : -1;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      row[u] = tile_row(&sm->rows, q0 + u * NT + (int)threadIdx.x, ne);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (t[u] >= 0 && c[u] == sm->comm[row[u]]) ex = __dadd_rn(ex, x[u]);
+  }
+}
+
 // Modularity partials of merge tile `tile` added to (ex, a2): a2 over the rows
 // that end in the tile, ex over its entries whose two ends share a community
 // (colour phases) or the rows' own_w (Jacobi phases).  All NT threads call.
@@ -284,23 +310,10 @@ __device__ __forceinline__ void modularity_merge_tile(int64_t tile, int64_t nv, 
   const int64_t ih = min(i1, nv - 1);
   const int nr = (int)(ih - i0 + 1);
   __syncthreads();  // the previous tile's readers are done
-  for (int k = threadIdx.x; k <= nr; k += NT) {
-    const int64_t r = ptr[i0 + k] - j0;
-    sm->off[k] = (int32_t)max((int64_t)0, min(r, (int64_t)kMergeTile + 1));
-  }
-  for (int k = threadIdx.x; k < nr; k += NT) sm->comm[k] = C[i0 + k];
-  __syncthreads();
   const int ne = (int)(j1 - j0);
-#pragma unroll 4
-  for (int q = threadIdx.x; q < ne; q += NT) {
-    int lo = 0, hi = nr - 1;  // the last row starting at or before q
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (sm->off[mid] <= q) lo = mid; else hi = mid - 1;
-    }
-    const int64_t e = j0 + q;
-    if (C[tail[e]] == sm->comm[lo]) ex = __dadd_rn(ex, w[e]);
-  }
+  for (int k = threadIdx.x; k < nr; k += NT) sm->comm[k] = C[i0 + k];
+  tile_rows_fill(&sm->rows, ptr, i0, nr, j0, ne);
+  modularity_entries<NT, NT == 256 ? 8 : 4>(j0, ne, tail, w, C, sm, ex);
 }
 
 // Batches of graphs: per-graph modularity sums {e_xx, a2_x} in gacc[2g],
@@ -348,21 +361,20 @@ __device__ __forceinline__ void modularity_merge_tile_graphs(
   const int64_t ih = min(i1, nv - 1);
   const int nr = (int)(ih - i0 + 1);
   __syncthreads();
-  for (int k = threadIdx.x; k <= nr; k += NT) {
-    const int64_t r = ptr[i0 + k] - j0;
-    sm->off[k] = (int32_t)max((int64_t)0, min(r, (int64_t)kMergeTile + 1));
-  }
-  for (int k = threadIdx.x; k < nr; k += NT) sm->comm[k] = C[i0 + k];
-  __syncthreads();
   const int ne = (int)(j1 - j0);
-  for (int q = threadIdx.x; q < ne; q += NT) {
-    int lo = 0, hi = nr - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (sm->off[mid] <= q) lo = mid; else hi = mid - 1;
-    }
-    const int64_t e = j0 + q;
-    if (C[tail[e]] == sm->comm[lo]) graph_acc_add(acc, gid[i0 + lo], w[e], 0.0, gacc);
+  for (int k = threadIdx.x; k < nr; k += NT) sm->comm[k] = C[i0 + k];
+  tile_rows_fill(&sm->rows, ptr, i0, nr, j0, ne);
+  if (gid[i0] == gid[ih]) {  // one graph's tile (block-uniform): no graph per entry
+    double ex = 0.0;
+    modularity_entries<NT, NT == 256 ? 8 : 4>(j0, ne, tail, w, C, sm, ex);
+    if (ex != 0.0) graph_acc_add(acc, gid[i0], ex, 0.0, gacc);
+    return;
+  }
+  for (int q0 = 0; q0 < ne; q0 += NT) {
+    const int q = q0 + (int)threadIdx.x;
+    const int lo = tile_row(&sm->rows, q, ne);
+    if (q < ne && C[tail[j0 + q]] == sm->comm[lo])
+      graph_acc_add(acc, gid[i0 + lo], w[j0 + q], 0.0, gacc);
   }
 }
 
@@ -409,23 +421,17 @@ __global__ void __launch_bounds__(256) k_step_pairs(int64_t nv, int64_t nnz, con
     const int64_t ih = min(i1, nv - 1);
     const int nr = (int)(ih - i0 + 1);
     __syncthreads();
-    for (int k = threadIdx.x; k <= nr; k += blockDim.x) {
-      const int64_t r = ptr[i0 + k] - j0;
-      sm.off[k] = (int32_t)max((int64_t)0, min(r, (int64_t)kMergeTile + 1));
-    }
     // the row's step, or -1 when the step is an independent set
     for (int k = threadIdx.x; k < nr; k += blockDim.x) {
       const int32_t st = step_of[i0 + k];
       sm.comm[k] = (st >= 0 && relaxed[st]) ? st : -1;
     }
-    __syncthreads();
     const int ne = (int)(j1 - j0);
-    for (int q = threadIdx.x; q < ne; q += blockDim.x) {
-      int lo = 0, hi = nr - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (sm.off[mid] <= q) lo = mid; else hi = mid - 1;
-      }
+    tile_rows_fill(&sm.rows, ptr, i0, nr, j0, ne);
+    for (int q0 = 0; q0 < ne; q0 += blockDim.x) {
+      const int q = q0 + (int)threadIdx.x;
+      const int lo = tile_row(&sm.rows, q, ne);
+      if (q >= ne) continue;
       const int32_t st = sm.comm[lo];
       if (st < 0) continue;
       const int64_t e = j0 + q;
@@ -719,24 +725,16 @@ __device__ __forceinline__ void coarse_tile(int64_t tile, int64_t nv, int64_t nn
     const int64_t ih = min(i1, nv - 1);
     const int nr = (int)(ih - i0 + 1);
     __syncthreads();
-    for (int k = threadIdx.x; k <= nr; k += blockDim.x) {
-      const int64_t r = ptr[i0 + k] - j0;
-      sm->off[k] = (int32_t)max((int64_t)0, min(r, (int64_t)kMergeTile + 1));
-    }
-    for (int k = threadIdx.x; k < nr; k += blockDim.x) sm->comm[k] = C[i0 + k];
-    __syncthreads();
     const int ne = (int)(j1 - j0);
+    for (int k = threadIdx.x; k < nr; k += blockDim.x) sm->comm[k] = C[i0 + k];
+    tile_rows_fill(&sm->rows, ptr, i0, nr, j0, ne);
     for (int q0 = 0; q0 < ne; q0 += blockDim.x) {  // block-uniform rounds
       const int q = q0 + (int)threadIdx.x;
       bool keep = false;
       uint64_t key = 0;
       int64_t e = 0;
+      const int lo = tile_row(&sm->rows, q, ne);
       if (q < ne) {
-        int lo = 0, hi = nr - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (sm->off[mid] <= q) lo = mid; else hi = mid - 1;
-        }
         e = j0 + q;
         const int32_t a = sm->comm[lo];
         const int32_t b = C[tail[e]];
