@@ -344,27 +344,17 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_sweep_iteration(IterArgs
       // warps numbered across blocks first: a step with few warp items spreads over SMs
       const int warp = thread_id() >> 5, ngw = gridDim.x * (kPersistThreads / 32);
       const int gwi = warp * gridDim.x + blockIdx.x;
-      const int i4 = (st.seg[1] - st.seg[0] + 7) / 8, i8 = (st.seg[2] - st.seg[1] + 3) / 4;
-      const int i16 = (st.seg[3] - st.seg[2] + 1) / 2;
-      const int witems = i4 + i8 + i16 + st.seg[5] - st.seg[3];
-      for (int k = gwi; k < witems; k += ngw) {
-        int q = k;
-        if (q < i4) { small_item<4>(p.a, st.seg[0] + 8 * q, st.seg[1]); continue; }
-        q -= i4;
-        if (q < i8) { small_item<8>(p.a, st.seg[1] + 4 * q, st.seg[2]); continue; }
-        q -= i8;
-        if (q < i16) { small_item<16>(p.a, st.seg[2] + 2 * q, st.seg[3]); continue; }
-        q -= i16 - st.seg[3];  // its member position
-        if (q < st.seg[4]) small_item<32>(p.a, q, st.seg[4]);
-        else
-          row_vertex<32>(p.a, q,
-                         tkeys + (warp >> 2) * kTeamCap + (warp & 3) * kPersistWarpCap,
-                         tvals + (warp >> 2) * kTeamCap + (warp & 3) * kPersistWarpCap,
-                         fill + (warp >> 2) * (kPersistFill * kTeamThreads / kPersistThreads) +
-                             (warp & 3) * 128,
-                         0, nullptr, nullptr, nullptr, nullptr);
-      }
-      GLV_QTRACE(s, 2, (threadIdx.x & 31) == 0 && gwi < witems);
+      int k = small_rows<4>(p.a, st.seg[0], st.seg[1], gwi, ngw);
+      k = small_rows<8>(p.a, st.seg[1], st.seg[2], k, ngw);
+      k = small_rows<16>(p.a, st.seg[2], st.seg[3], k, ngw);
+      k = small_rows<32>(p.a, st.seg[3], st.seg[4], k, ngw);
+      for (int pos = st.seg[4] + k; pos < st.seg[5]; pos += ngw)
+        row_vertex<32>(p.a, pos, tkeys + (warp >> 2) * kTeamCap + (warp & 3) * kPersistWarpCap,
+                       tvals + (warp >> 2) * kTeamCap + (warp & 3) * kPersistWarpCap,
+                       fill + (warp >> 2) * (kPersistFill * kTeamThreads / kPersistThreads) +
+                           (warp & 3) * 128,
+                       0, nullptr, nullptr, nullptr, nullptr);
+      GLV_QTRACE(s, 2, (threadIdx.x & 31) == 0);
     }
     __syncthreads();
     if (thread_id() == 0 && block_moved()) {

@@ -214,4 +214,143 @@ __device__ __forceinline__ void row_vertex(const SweepArgs &a, int64_t pos, int3
   if (NW == 1) __syncwarp();
 }
 
+// ---------------------------------------------------------------------------
+// Rows of at most 32 entries: G lanes per row, 32 / G rows per warp and item,
+// everything in registers.  A warp runs its items of a bin one after another
+// (item k, k + stride, ...), and an item is a chain of four dependent loads
+// (member, row bounds, entries, communities), so the loads run ahead: while an
+// item is decided, the next one's entries, the one after's row bounds and the
+// third's members are on their way.
+struct SmallRow {
+  int32_t v;       // -1: no row
+  int deg;
+  int64_t rb;
+};
+
+__device__ __forceinline__ void small_bounds(const SweepArgs &a, SmallRow &r) {
+  r.rb = 0;
+  r.deg = 0;
+  if (r.v >= 0) {
+    r.rb = a.ptr[r.v];
+    r.deg = (int)(a.ptr[r.v + 1] - r.rb);
+  }
+}
+
+// Decides the 32 / G rows of an item: row r, entry (t, w) of this lane, own =
+// community of r.v (-1 for an empty row).
+template <int G>
+__device__ __forceinline__ void small_decide(const SweepArgs &a, int pos, const SmallRow &r,
+                                             int32_t t, double w, int32_t own) {
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+  const bool skip = r.deg > 0 && skipped(a, r.v);
+  const bool has = !skip && gl < r.deg;
+  const int32_t c = has ? a.C[t] : -1;
+  // the community's and the vertex's totals, while the entries are compared
+  const double degree = r.deg > 0 ? a.vDeg[r.v] : 0.0;
+  const double cdeg_own = r.deg > 0 ? a.cDeg[own] : 0.0;
+  const double cdeg = (has && c != own) ? a.cDeg[c] : 0.0;
+  const int32_t own_size = (r.deg > 0 && gl == 0) ? a.cSize[own] : 0;
+  double sum, own_w = 0.0, self_w = 0.0;  // Counter[c], Counter[own], self-loops
+  bool cand;                              // this lane offers community c
+  if (G <= 8) {
+    // every lane sees the other lanes of its row in turn (3 shuffles each; a
+    // match over the warp takes up to 379 cycles); the top bit marks self-loops
+    const int32_t mark = (has && t == r.v) ? (c | INT32_MIN) : (has ? c : 0x7fffffff);
+    sum = has ? w : 0.0;
+    if (c == own && has) own_w = w;
+    if (has && t == r.v) self_w = w;
+#pragma unroll
+    for (int off = 1; off < G; ++off) {
+      const int src = (lane & ~(G - 1)) | ((gl + off) & (G - 1));
+      const int32_t oc = __shfl_sync(FULL, mark, src);
+      const double ow = __shfl_sync(FULL, w, src);
+      const int32_t id = oc & 0x7fffffff;
+      if (id == c) sum = __dadd_rn(sum, ow);
+      if (id == own) own_w = __dadd_rn(own_w, ow);
+      if (oc < 0) self_w = __dadd_rn(self_w, ow);
+    }
+    cand = has && c != own;
+  } else {
+    const unsigned gmask = (G == 32) ? FULL : (((1u << (G & 31)) - 1u) << (lane & ~(G - 1)));
+    const unsigned m = __match_any_sync(FULL, c) & gmask;
+    sum = group_sum(has ? w : 0.0, has ? m : 0u);
+    const bool leader = has && lane == __ffs(m) - 1;
+    const unsigned om = __ballot_sync(FULL, leader && c == own) & gmask;
+    own_w = __shfl_sync(FULL, sum, om ? __ffs(om) - 1 : lane);
+    if (!om) own_w = 0.0;
+    const unsigned sm = __ballot_sync(FULL, has && t == r.v) & gmask;
+    if (__any_sync(FULL, sm != 0)) {
+      self_w = group_sum((has && t == r.v) ? w : 0.0, (has && t == r.v) ? sm : 0u);
+      self_w = __shfl_sync(FULL, self_w, sm ? __ffs(sm) - 1 : lane);
+      if (!sm) self_w = 0.0;
+    }
+    cand = leader && c != own;
+  }
+  double g = 0.0;
+  int32_t bc = INT32_MAX;
+  if (cand) {
+    const double eix = __dsub_rn(own_w, self_w);
+    const double ax = __dsub_rn(cdeg_own, degree);
+    const double gain = louvain_gain(sum, eix, degree, cdeg, ax, cst_of(a, r.v));
+    if (gain > 0.0) { g = gain; bc = c; }
+  }
+#pragma unroll
+  for (int off = G / 2; off >= 1; off >>= 1) {
+    const double og = __shfl_xor_sync(FULL, g, off);
+    const int32_t oc = __shfl_xor_sync(FULL, bc, off);
+    if (better(og, oc, g, bc)) { g = og; bc = oc; }
+  }
+  if (r.v >= 0 && gl == 0) {
+    if (skip) {
+      emit_stay(a, pos, r.v, own);
+    } else {
+      const int32_t tgt = (r.deg == 0) ? -1 : finish_choice(a, own, own_size, g, bc);
+      emit_decision(a, pos, r.v, own, tgt, degree, own_w, g);
+    }
+  }
+}
+
+// This warp's items k, k + stride, ... of the rows at member positions
+// [begin, end); returns the first item number past the bin's, for the next bin.
+template <int G>
+__device__ __forceinline__ int small_rows(const SweepArgs &a, int begin, int end, int k,
+                                          int stride) {
+  constexpr int VPW = 32 / G;
+  const int n = (end - begin + VPW - 1) / VPW;
+  if (k < n) {
+    const int grp = (threadIdx.x & 31) / G, gl = threadIdx.x & (G - 1);
+    const int hop = VPW * stride;
+    int pos = begin + VPW * k + grp;
+    SmallRow cur, nxt;
+    cur.v = (pos < end) ? a.members[pos] : -1;
+    nxt.v = (pos + hop < end) ? a.members[pos + hop] : -1;
+    int32_t v3 = (pos + 2 * hop < end) ? a.members[pos + 2 * hop] : -1;
+    small_bounds(a, cur);
+    small_bounds(a, nxt);
+    int32_t t = (gl < cur.deg) ? __ldcs(&a.tail[cur.rb + gl]) : -1;
+    double w = (gl < cur.deg) ? __ldcs(&a.w[cur.rb + gl]) : 0.0;
+    int32_t own = cur.deg > 0 ? a.C[cur.v] : -1;
+    for (;;) {
+      // ahead: the next item's entries, the one after's bounds, a third's members
+      const int32_t t2 = (gl < nxt.deg) ? __ldcs(&a.tail[nxt.rb + gl]) : -1;
+      const double w2 = (gl < nxt.deg) ? __ldcs(&a.w[nxt.rb + gl]) : 0.0;
+      const int32_t own2 = nxt.deg > 0 ? a.C[nxt.v] : -1;
+      SmallRow after;
+      after.v = v3;
+      small_bounds(a, after);
+      v3 = (pos + 3 * hop < end) ? a.members[pos + 3 * hop] : -1;
+      small_decide<G>(a, pos, cur, t, w, own);
+      k += stride;
+      if (k >= n) break;
+      pos += hop;
+      cur = nxt;
+      nxt = after;
+      t = t2;
+      w = w2;
+      own = own2;
+    }
+  }
+  return k - n;
+}
+
 }  // namespace glv
