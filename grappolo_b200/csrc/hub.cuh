@@ -5,7 +5,7 @@
 //              then written out as (community, weight) pairs grouped by
 //              partition (mix32(community) mod nparts) with the partitions'
 //              offsets.  The block that finishes a hub's last chunk merges all
-//              pairs and decides the hub when they are few (kHubInline);
+//              pairs and decides the hub when they are few (inline_pairs);
 //   partition  one partition's pairs of all the hub's chunks, merged in the
 //              block's shared table and scanned for the best gain; the last
 //              partition to finish folds the partitions' bests and decides.
@@ -25,19 +25,21 @@ namespace glv {
 constexpr int kHubThreads = 512;
 constexpr int kHubTableCap = 8192;   // the block's table
 constexpr int kHubList = 4096;       // filled slots a merge may hold at once
-constexpr int kHubInline = 2048;     // pairs the last chunk's block merges itself
+constexpr int kHubInline = 2048;     // pairs the last chunk's block merges itself; in full
+constexpr int kHubInlineFull = 4096; // steps (HubInfo::inline_pairs)
 constexpr int kHubMaxParts = 512;
-constexpr int kHubPartEntries = 1024;  // row entries per partition (more only past kHubMaxParts)
 constexpr int kHubRuns = 512;        // chunks a merge looks up at a time
 constexpr uint32_t kSpinLimit = 1u << 22;  // polls of a partition's wait (>= 128 ns each)
+static_assert(kHubInlineFull <= kHubList, "an inline merge fits the list");
 static_assert(kHubChunk <= 2048 && kHubChunk <= kHubTableCap / 2, "a chunk fits the table");
 static_assert(kHubRuns <= kHubThreads && kHubRuns <= kHubMaxParts, "one thread per run");
 static_assert(kHubChunk < 65536 && kHubTableCap <= kNoSlot, "16-bit offsets and slots");
 
-// Partitions of a row (a power of two, at least 2).
-__host__ __device__ inline int hub_parts(int64_t deg) {
+// Partitions of a row (a power of two, at least 2) of about `entries` row
+// entries each (more only past kHubMaxParts).
+__host__ __device__ inline int hub_parts(int64_t deg, int entries) {
   int p = 2;
-  while (p < kHubMaxParts && (int64_t)p * kHubPartEntries < deg) p <<= 1;
+  while (p < kHubMaxParts && (int64_t)p * entries < deg) p <<= 1;
   return p;
 }
 
@@ -283,7 +285,7 @@ __device__ __forceinline__ void hub_chunk_task(const SweepArgs &a, const HubWork
     }
     return;
   }
-  if (__ldcg(&hs->cnt) > kHubInline) {
+  if (__ldcg(&hs->cnt) > hb.inline_pairs) {
     if (threadIdx.x == 0) atomicExch(&hs->state, decided + 1u);  // its partitions decide it
     return;
   }

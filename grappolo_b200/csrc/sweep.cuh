@@ -466,6 +466,7 @@ struct HubInfo {
   int32_t pos;              // member slot
   int32_t chunk0, nchunks;  // its chunks
   int32_t part0, nparts;    // its partitions (nparts a power of two)
+  int32_t inline_pairs;     // most pairs the last chunk's block merges itself
 };
 struct HubChunk {
   int64_t beg;              // CSR range [beg, beg + len)
