@@ -23,6 +23,7 @@
 #include "batch_kernels.cuh"
 #include "color_flow.cuh"
 #include "gate.cuh"
+#include "ordered.cuh"
 #include "persist.cuh"
 #include "recolor.cuh"
 #include "vbase.cuh"
@@ -1511,6 +1512,32 @@ constexpr int kBlockCap = 8192; // table_cap(4095)
 int Engine::launch_sweep(const Level &L, const Step &st, SweepArgs a, bool ordered_acc,
                          Probes *pr) {
   const int cap = nsm_ * 16;
+  if (ordered_acc) {
+    // one launch for all bins, or one per bin when each launch is timed
+    const bool split = pr && pr->level >= 2;
+    for (int first = 0; first < NBINS; ++first) {
+      BinRanges r{};
+      int64_t nlong = 0, items = 0;
+      constexpr int vpw[NBINS] = {8, 4, 2, 1, 1, 0, 0, 0, 0};
+      for (int b = first; b < (split ? first + 1 : NBINS); ++b) {
+        r.lo[b] = st.seg[b];
+        r.hi[b] = st.seg[b + 1];
+        const int64_t n = r.hi[b] - r.lo[b];
+        if (b >= BIN_T128) nlong += n;
+        else items += (n + vpw[b] - 1) / vpw[b];
+      }
+      if (nlong + items > 0) {
+        int pidx = -1;
+        if (pr) TRY(pr->begin(first, 2, s_, &pidx));
+        const int gl = (int)std::min<int64_t>(nlong, nsm_);
+        const int gw = (int)std::min<int64_t>((items + kOrdWarps - 1) / kOrdWarps, nsm_ * 2);
+        LAUNCH(k_sweep_ordered, gl + gw, kOrdThreads, kOrdSmem, s_, a, r, gl);
+        if (pr) TRY(pr->end(pidx, s_));
+      }
+      if (!split) break;
+    }
+    return GLV_OK;
+  }
   for (int b = 0; b < NBINS; ++b) {
     const int64_t lo = st.seg[b], hi = st.seg[b + 1];
     const int64_t n = hi - lo;
@@ -1539,23 +1566,19 @@ int Engine::launch_sweep(const Level &L, const Step &st, SweepArgs a, bool order
       case BIN_T256:
       case BIN_BLOCK: {
         const size_t smem = (size_t)kBlockCap * (sizeof(double) + sizeof(int32_t));
-        LAUNCH(k_sweep_block, (int)std::min<int64_t>(n, nsm_ * 2), 256, smem, s_, a, lo, hi, 0,
-               ordered_acc ? 1 : 0);
+        LAUNCH(k_sweep_block, (int)std::min<int64_t>(n, nsm_ * 2), 256, smem, s_, a, lo, hi);
         break;
       }
-      case BIN_HUB:
-        if (ordered_acc) {
-          LAUNCH(k_sweep_block, (int)std::min<int64_t>(n, nsm_), 512, 0, s_, a, lo, hi, 1, 1);
-        } else {
-          const HubWork hw = hub_work();
-          const int64_t nc = st.hub_chunk[1] - st.hub_chunk[0];
-          const int64_t ns = st.hub_segs[1] - st.hub_segs[0];
-          LAUNCH(k_hub_tasks<false>, (int)std::min<int64_t>(nc, nsm_ * 2), kHubThreads, kHubSmem,
-                 s_, a, hw, st.hub_chunk[0], st.hub_chunk[1]);
-          LAUNCH(k_hub_tasks<true>, (int)std::min<int64_t>(ns, nsm_ * 2), kHubThreads, kHubSmem,
-                 s_, a, hw, st.hub_segs[0], st.hub_segs[1]);
-        }
+      case BIN_HUB: {
+        const HubWork hw = hub_work();
+        const int64_t nc = st.hub_chunk[1] - st.hub_chunk[0];
+        const int64_t ns = st.hub_segs[1] - st.hub_segs[0];
+        LAUNCH(k_hub_tasks<false>, (int)std::min<int64_t>(nc, nsm_ * 2), kHubThreads, kHubSmem,
+               s_, a, hw, st.hub_chunk[0], st.hub_chunk[1]);
+        LAUNCH(k_hub_tasks<true>, (int)std::min<int64_t>(ns, nsm_ * 2), kHubThreads, kHubSmem,
+               s_, a, hw, st.hub_segs[0], st.hub_segs[1]);
         break;
+      }
     }
     if (pr) TRY(pr->end(pidx, s_));
   }
@@ -1567,6 +1590,11 @@ int Engine::launch_apply(const ClassSched &cs, bool ordered_upd) {
   if (!ordered_upd) {
     LAUNCH(k_apply_deltas, grid_for(n, 256, nsm_ * 16), 256, 0, s_, cs.begin, cs.end, move_old_,
            move_new_, dDeg, dSize, cDeg, cSize);
+    return GLV_OK;
+  }
+  if (n <= kOrdApplyMax) {
+    LAUNCH(k_apply_ordered, 1, kOrdApplyThreads, kOrdApplySmem, s_, cs.begin, cs.end, members_,
+           move_old_, move_new_, vDeg, cDeg, cSize);
     return GLV_OK;
   }
   const uint64_t sentinel = (uint64_t)(uint32_t)nv0_ << 32;
@@ -3382,6 +3410,8 @@ static int set_kernel_attributes() {
       {(const void *)k_hc_tiles, (int)sizeof(HashTileSmem)},
       {(const void *)k_row_sums_tiles, (int)sizeof(RowSumSmem)},
       {(const void *)k_flow_counts, (int)sizeof(FlowTileSmem)},
+      {(const void *)k_sweep_ordered, kOrdSmem},
+      {(const void *)k_apply_ordered, kOrdApplySmem},
   };
   for (const auto &k : want) {
     const cudaError_t e =

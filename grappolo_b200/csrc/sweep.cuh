@@ -380,13 +380,12 @@ __global__ void __launch_bounds__(256) k_sweep_warp(SweepArgs a, int64_t begin, 
 }
 
 // ---------------------------------------------------------------------------
-// Large rows: one block per vertex; the table is `keys`/`vals` (shared memory
-// or a global region).  ordered = 1: warp 0 walks the whole row in CSR order
-// (bit-exact sums); ordered = 0: all warps take chunks and add group sums with
-// atomics.  `red` is block scratch of 3 x 32 words.  All threads call.
+// Large rows without the persistent kernel (parallel accumulation): one block
+// per vertex, the table in shared memory; all warps take rounds of 32 entries
+// and add group sums with atomics.  All threads call.
 __device__ __forceinline__ void block_vertex(const SweepArgs &a, int64_t pos, int32_t *keys,
-                                             double *vals, int ordered, double *s_self,
-                                             double *s_g, int32_t *s_c) {
+                                             double *vals, double *s_self, double *s_g,
+                                             int32_t *s_c) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int nwb = blockDim.x >> 5;
@@ -399,21 +398,12 @@ __device__ __forceinline__ void block_vertex(const SweepArgs &a, int64_t pos, in
   const int32_t own = a.C[v];
   if (threadIdx.x == 0) keys[hash_slot(own, mask)] = own;
   __syncthreads();
-  double self_loop;
-  if (ordered) {
-    if (warp == 0) {
-      double sl = warp_accumulate(a, v, rb, re, 32, keys, vals, mask, false);
-      if (lane == 0) s_self[0] = sl;
-    }
-    __syncthreads();
-    self_loop = s_self[0];
-  } else {
-    double sl = warp_accumulate(a, v, rb + 32 * warp, re, 32 * nwb, keys, vals, mask, true);
-    if (lane == 0) s_self[warp] = sl;
-    __syncthreads();
-    self_loop = 0.0;
-    for (int k = 0; k < nwb; ++k) self_loop = __dadd_rn(self_loop, s_self[k]);
-  }
+  const double sl =
+      warp_accumulate(a, v, rb + 32 * warp, re, 32 * nwb, keys, vals, mask, true);
+  if (lane == 0) s_self[warp] = sl;
+  __syncthreads();
+  double self_loop = 0.0;
+  for (int k = 0; k < nwb; ++k) self_loop = __dadd_rn(self_loop, s_self[k]);
   const double degree = a.vDeg[v];
   const double own_w = vals[hash_slot(own, mask)];
   const double eix = __dsub_rn(own_w, self_loop);
@@ -432,27 +422,17 @@ __device__ __forceinline__ void block_vertex(const SweepArgs &a, int64_t pos, in
   __syncthreads();
 }
 
-// BIN_T128/T256/BLOCK keep the table in shared memory (capacity up to 8192),
-// BIN_HUB in global scratch at hub_off.
-__global__ void __launch_bounds__(512) k_sweep_block(SweepArgs a, int64_t begin, int64_t end,
-                                                     int hub, int ordered) {
+__global__ void __launch_bounds__(512) k_sweep_block(SweepArgs a, int64_t begin, int64_t end) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ double s_self[32];
   __shared__ double s_g[32];
   __shared__ int32_t s_c[32];
   for (int64_t pos = begin + blockIdx.x; pos < end; pos += gridDim.x) {
-    int32_t *keys;
-    double *vals;
-    if (hub) {
-      keys = a.hub_keys + a.hub_off[pos];
-      vals = a.hub_vals + a.hub_off[pos];
-    } else {
-      const int32_t v = a.members[pos];
-      const uint32_t cap = table_cap(a.ptr[v + 1] - a.ptr[v]);
-      vals = reinterpret_cast<double *>(smem_raw);
-      keys = reinterpret_cast<int32_t *>(vals + cap);
-    }
-    block_vertex(a, pos, keys, vals, ordered, s_self, s_g, s_c);
+    const int32_t v = a.members[pos];
+    const uint32_t cap = table_cap(a.ptr[v + 1] - a.ptr[v]);
+    double *vals = reinterpret_cast<double *>(smem_raw);
+    int32_t *keys = reinterpret_cast<int32_t *>(vals + cap);
+    block_vertex(a, pos, keys, vals, s_self, s_g, s_c);
   }
 }
 
