@@ -17,7 +17,9 @@
 //    stable-sorted by row, which is the loaders' fill order;
 //  * sorted rows: the reference's bottom-up merge takes the right run on equal
 //    tails, so equal tails end in descending position; a stable sort by
-//    (row, tail) of the entries listed in reverse gives exactly that.
+//    (row, tail) of the entries listed in reverse gives exactly that;
+//  * both at once: sorted rows are merged from the kept edges as they stand
+//    (by head) and sorted by tail.
 //
 // Included into engine.cu after the C ABI helpers (Call, fail, CK, TRY).
 
@@ -364,6 +366,327 @@ static int row_entries(cudaStream_t s, int64_t nv, int64_t nk, const int64_t *or
   return GLV_OK;
 }
 
+// ---- removeEdges and sorted rows together --------------------------------
+// The sort that finds repeats leaves the kept edges in (head, tail) order, which
+// is the order of their head-side entries.  Their tail-side entries need only a
+// stable sort of that list on the tail's bits (half the passes over half the
+// records of a new sort of all directed entries), and the rows are the merge of
+// the two lists: both are ordered by (row, column) over the whole graph.
+// R-MAT 22 (67M edges): 15.7 ms by sorting all entries anew, 9.15 this way, of
+// which the two sorts 5.1, the weights' gathers 1.7, the rest of the merge 1.2.
+//
+// Equal entries come latest first, by the slots removeEdges leaves the edges in:
+// an edge below NGE keeps its slot, and the q-th kept edge from NGE on fills the
+// q-th hole from the end.  Only ties need slots, so only the dropped places are
+// kept, in order: the holes are those below NGE.
+struct KeptSorted {
+  int64_t nge = 0, ndrop = 0;
+  uint64_t *key = nullptr;   // kept edges by (head, tail): head << bits | tail
+  int32_t *idx = nullptr;    // their places in the list
+  int32_t *drop = nullptr;   // dropped places, ascending
+};
+
+constexpr int kPickItems = 8;            // records a lane of k_pick
+constexpr int kPickTile = 256 * kPickItems;
+constexpr int kRunItems = 7;  // entries a thread of k_merge_runs; odd: the threads'
+constexpr int kRunThreads = 256;
+constexpr int kRunTile = kRunThreads * kRunItems;  // runs start in different banks
+
+__global__ void k_pair_keys32(int64_t ne, EdgeView ev, int64_t nv, int bits, uint64_t *keys,
+                              int32_t *idx, int32_t *bad) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ne;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    int64_t h = ev.h(i), t = ev.t(i);
+    if (h < 0 || h >= nv || t < 0 || t >= nv) {
+      atomicOr(bad, 1);
+      h = t = 0;
+    }
+    keys[i] = ((uint64_t)h << bits) | (uint64_t)t;
+    idx[i] = (int32_t)i;
+  }
+}
+
+// Whether sorted record s is the first of its (head, tail) run and no self-loop.
+__device__ __forceinline__ bool run_first(const uint64_t *skeys, int64_t s, int bits, uint64_t k) {
+  return (k >> bits) != (k & ((1ull << bits) - 1)) && (s == 0 || skeys[s - 1] != k);
+}
+
+// One block per tile of sorted records.  idx null: kept[tile] = its kept
+// records; otherwise they go to key / idx from kept[tile] (the tile's offset)
+// on, in order, and the other records' places to drop.  A warp takes 256
+// records in a row, so its writes are coalesced (two passes over the keys,
+// 8 + 24 bytes a record, 0.58 ms for 67M; a scatter of one flag byte per record
+// to its place in the list and selections from those flags took 1.3).
+template <bool kWrite>
+__global__ void __launch_bounds__(256) k_pick(int64_t ne, int bits, const uint64_t *skeys,
+                                              const int32_t *sidx, int64_t *kept, uint64_t *key,
+                                              int32_t *idx, int32_t *drop) {
+  __shared__ int s_n[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t s0 = (int64_t)blockIdx.x * kPickTile + warp * (32 * kPickItems);
+  uint64_t k[kPickItems];
+  unsigned m[kPickItems];
+  int n = 0;
+#pragma unroll
+  for (int u = 0; u < kPickItems; ++u) {
+    const int64_t s = s0 + u * 32 + lane;
+    k[u] = s < ne ? skeys[s] : 0;
+    m[u] = __ballot_sync(0xffffffffu, s < ne && run_first(skeys, s, bits, k[u]));
+    n += __popc(m[u]);
+  }
+  if (lane == 0) s_n[warp] = n;
+  __syncthreads();
+  int before = 0, all = 0;
+  for (int w = 0; w < 8; ++w) {
+    if (w < warp) before += s_n[w];
+    all += s_n[w];
+  }
+  if constexpr (!kWrite) {
+    if (threadIdx.x == 0) kept[blockIdx.x] = all;
+  } else {
+    int64_t at = kept[blockIdx.x] + before;
+#pragma unroll
+    for (int u = 0; u < kPickItems; ++u) {
+      const int64_t s = s0 + u * 32 + lane;
+      const int64_t p = at + __popc(m[u] & ((1u << lane) - 1));
+      at += __popc(m[u]);
+      if (s >= ne) continue;
+      if (m[u] >> lane & 1) {
+        key[p] = k[u];
+        idx[p] = sidx[s];
+      } else {
+        drop[s - p] = sidx[s];
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ int64_t drops_below(const KeptSorted &ks, int64_t place) {
+  int64_t lo = 0, hi = ks.ndrop;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (ks.drop[mid] < place) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+// The slot that removeEdges leaves the kept list edge i in.
+__device__ __forceinline__ int64_t kept_slot(const KeptSorted &ks, int32_t i) {
+  if (i < ks.nge) return i;
+  const int64_t holes = drops_below(ks, ks.nge);
+  const int64_t q = (i - ks.nge) - (drops_below(ks, i) - holes);
+  return ks.drop[holes - 1 - q];
+}
+
+// The two lists of directed entries: by head as the kept edges stand, by tail
+// as sorted on the tail's bits (still head << bits | tail).
+struct EntryRuns {
+  KeptSorted ks;
+  const uint64_t *tkey;
+  const int32_t *tidx;
+  int bits;
+  __device__ __forceinline__ uint64_t tail_side(int64_t j) const {
+    const uint64_t k = tkey[j];
+    return ((k & ((1ull << bits) - 1)) << bits) | (k >> bits);
+  }
+};
+
+// Whether the head-side entry (ka, edge ia) comes before the tail-side (kb, ib).
+__device__ __forceinline__ bool head_first(const KeptSorted &ks, uint64_t ka, uint64_t kb,
+                                           int32_t ia, int32_t ib) {
+  return ka != kb ? ka < kb : kept_slot(ks, ia) > kept_slot(ks, ib);
+}
+
+// split[t] = head-side entries among the first t * kRunTile merged ones.
+__global__ void k_run_splits(EntryRuns r, int64_t ntiles, int64_t *split) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t > ntiles) return;
+  const int64_t n = r.ks.nge, d = min(t * (int64_t)kRunTile, 2 * n);
+  int64_t lo = max((int64_t)0, d - n), hi = min(d, n);
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1, j = d - 1 - mid;
+    if (head_first(r.ks, r.ks.key[mid], r.tail_side(j), r.ks.idx[mid], r.tidx[j]))
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  split[t] = lo;
+}
+
+// One tile of the merged entries per block: both lists' parts to shared memory,
+// each thread merges kRunItems entries, and the merged tile is written out
+// coalesced, with the row offsets.  The weights are gathered by the edge's
+// place in the list, which is what bounds it (32-byte sectors for 8 bytes): 2.9
+// ms for 131M entries, 1.2 of it without weights.  Tiles of 3 to 7 entries a
+// thread and 128 or 256 threads measure the same to 1%, 11 and 15 entries 24%
+// more of the whole build.  A search of every entry in the other list's row
+// took 5.9 ms.
+__global__ void __launch_bounds__(kRunThreads) k_merge_runs(EntryRuns r, EdgeView ev, int64_t nv,
+                                                    const int64_t *split, int64_t *ptr,
+                                                    int32_t *otail, double *ow, glv_edge *oaos) {
+  __shared__ uint64_t s_key[kRunTile];
+  __shared__ int32_t s_idx[kRunTile];
+  __shared__ uint16_t s_from[kRunTile];  // where the merged tile's entries stand
+  const int64_t m = 2 * r.ks.nge;
+  const int64_t d0 = (int64_t)blockIdx.x * kRunTile;
+  const int n = (int)min((int64_t)kRunTile, m - d0);
+  const int64_t a0 = split[blockIdx.x], b0 = d0 - a0;
+  const int na = (int)(split[blockIdx.x + 1] - a0), nb = n - na;
+  const int bits = r.bits;
+#pragma unroll
+  for (int u = 0; u < kRunItems; ++u) {
+    const int q = u * kRunThreads + threadIdx.x;
+    if (q < na) {
+      s_key[q] = r.ks.key[a0 + q];
+      s_idx[q] = r.ks.idx[a0 + q];
+    } else if (q < n) {
+      s_key[q] = r.tail_side(b0 + q - na);
+      s_idx[q] = r.tidx[b0 + q - na];
+    }
+  }
+  __syncthreads();
+  const int d = min((int)threadIdx.x * kRunItems, n);
+  int lo = max(0, d - nb), hi = min(d, na);
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1, j = na + d - 1 - mid;
+    if (head_first(r.ks, s_key[mid], s_key[j], s_idx[mid], s_idx[j])) lo = mid + 1; else hi = mid;
+  }
+  int a = lo, b = na + d - lo;
+  uint64_t ka = a < na ? s_key[a] : ~0ull, kb = b < n ? s_key[b] : ~0ull;  // ~0: after any key
+#pragma unroll
+  for (int u = 0; u < kRunItems; ++u) {
+    if (d + u < n) {
+      const bool left = ka != kb ? ka < kb : head_first(r.ks, ka, kb, s_idx[a], s_idx[b]);
+      s_from[d + u] = (uint16_t)(left ? a : b);
+      if (left) {
+        ++a;
+        ka = a < na ? s_key[a] : ~0ull;
+      } else {
+        ++b;
+        kb = b < n ? s_key[b] : ~0ull;
+      }
+    }
+  }
+  __syncthreads();
+  double w[kRunItems];
+#pragma unroll
+  for (int u = 0; u < kRunItems; ++u) {
+    const int q = u * kRunThreads + threadIdx.x;
+    w[u] = q < n ? ev.wt(s_idx[s_from[q]]) : 0;
+  }
+  const uint64_t low = (1ull << bits) - 1;
+#pragma unroll
+  for (int u = 0; u < kRunItems; ++u) {
+    const int q = u * kRunThreads + threadIdx.x;
+    if (q >= n) continue;
+    const int64_t at = d0 + q;
+    const uint64_t k = s_key[s_from[q]];
+    const int64_t row = (int64_t)(k >> bits), col = (int64_t)(k & low);
+    if (otail) otail[at] = (int32_t)col;
+    if (ow) ow[at] = w[u];
+    if (oaos) oaos[at] = glv_edge{(long)row, (long)col, w[u]};
+    int64_t prev = -1;  // the row of the entry before
+    if (q > 0) {
+      prev = (int64_t)(s_key[s_from[q - 1]] >> bits);
+    } else {
+      if (a0 > 0) prev = (int64_t)(r.ks.key[a0 - 1] >> bits);
+      if (b0 > 0) prev = max(prev, (int64_t)(r.tail_side(b0 - 1) >> bits));
+    }
+    for (int64_t x = prev + 1; x <= row; ++x) ptr[x] = at;
+    if (at == m - 1)
+      for (int64_t x = row + 1; x <= nv; ++x) ptr[x] = m;
+  }
+}
+
+// Whether a build takes this way: both options, and list places in 32 bits.  It
+// is the faster one at every size measured: 128 edges 147 -> 138 us, 130k 285 ->
+// 249, 8M 2036 -> 1254, 67M 15700 -> 9150.
+static bool merges_rows(int flags, int64_t ne) {
+  return ne > 0 && ne < (int64_t(1) << 31) - 1 && (flags & GLV_CSR_REMOVE_EDGES) &&
+         (flags & GLV_CSR_SORT_ROWS);
+}
+
+static bool overlap(const void *a, int64_t na, const void *b, int64_t nb) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return a && b && x < y + (uintptr_t)nb && y < x + (uintptr_t)na;
+}
+
+// The kept edges in (head, tail) order.
+static int kept_sorted(cudaStream_t s, int64_t nv, int64_t ne, EdgeView ev, DevScratch &d,
+                       KeptSorted *ks, long *launches) {
+  uint64_t *k1, *k2;
+  int32_t *v1, *v2, *bad;
+  int64_t *cnt;
+  const int64_t tiles = (ne + kPickTile - 1) / kPickTile;
+  TRY(d.get(&k1, ne)); TRY(d.get(&k2, ne)); TRY(d.get(&v1, ne)); TRY(d.get(&v2, ne));
+  TRY(d.get(&bad, 1)); TRY(d.get(&cnt, tiles + 1));
+  CK(cudaMemsetAsync(bad, 0, sizeof(int32_t), s));
+  CK(cudaMemsetAsync(cnt + tiles, 0, sizeof(int64_t), s));
+  const int bits = id_bits(nv);
+  k_pair_keys32<<<csr_grid(ne), 256, 0, s>>>(ne, ev, nv, bits, k1, v1, bad);
+  CK(cudaGetLastError());
+  size_t tb = 0, t2 = 0;
+  CK(cub::DeviceRadixSort::SortPairs(nullptr, tb, k1, k2, v1, v2, ne, 0, 2 * bits, s));
+  CK(cub::DeviceScan::ExclusiveSum(nullptr, t2, cnt, cnt, tiles + 1, s));
+  void *temp;
+  TRY(d.get((char **)&temp, (int64_t)std::max(tb, t2)));
+  CK(cub::DeviceRadixSort::SortPairs(temp, tb, k1, k2, v1, v2, ne, 0, 2 * bits, s));
+  k_pick<false><<<(unsigned)tiles, 256, 0, s>>>(ne, bits, k2, v2, cnt, nullptr, nullptr, nullptr);
+  CK(cudaGetLastError());
+  CK(cub::DeviceScan::ExclusiveSum(temp, t2, cnt, cnt, tiles + 1, s));
+  int32_t hbad = 0;
+  CK(cudaMemcpyAsync(&hbad, bad, sizeof(hbad), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(&ks->nge, cnt + tiles, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  if (hbad) return fail(GLV_ERR_ARG, "an edge end is outside [0, NV)");
+  ks->key = k1;
+  ks->idx = v1;
+  ks->ndrop = ne - ks->nge;
+  int32_t *drop = nullptr, *order = nullptr;
+  TRY(d.get(&drop, ks->ndrop)); TRY(d.get(&order, ks->ndrop));
+  k_pick<true><<<(unsigned)tiles, 256, 0, s>>>(ne, bits, k2, v2, cnt, k1, v1, drop);
+  CK(cudaGetLastError());
+  *launches += 3;
+  ks->drop = order;
+  if (ks->ndrop > 0 && ks->nge > 0) {
+    const int pb = id_bits(ne);
+    CK(cub::DeviceRadixSort::SortKeys(nullptr, t2, drop, order, ks->ndrop, 0, pb, s));
+    TRY(d.get((char **)&temp, (int64_t)t2));
+    CK(cub::DeviceRadixSort::SortKeys(temp, t2, drop, order, ks->ndrop, 0, pb, s));
+  }
+  return GLV_OK;
+}
+
+// The CSR of the kept edges, both directions, rows sorted.
+static int merged_rows(cudaStream_t s, int64_t nv, const KeptSorted &ks, EdgeView ev,
+                       DevScratch &d, int64_t *d_ptr, int32_t *otail, double *ow, glv_edge *oaos,
+                       long *launches) {
+  const int64_t n = ks.nge;
+  if (n == 0) {
+    CK(cudaMemsetAsync(d_ptr, 0, (nv + 1) * sizeof(int64_t), s));
+  } else {
+    EntryRuns r{ks, nullptr, nullptr, id_bits(nv)};
+    const int64_t tiles = (2 * n + kRunTile - 1) / kRunTile;
+    uint64_t *tkey;
+    int32_t *tidx;
+    int64_t *split;
+    TRY(d.get(&tkey, n)); TRY(d.get(&tidx, n)); TRY(d.get(&split, tiles + 1));
+    size_t tb = 0;
+    CK(cub::DeviceRadixSort::SortPairs(nullptr, tb, ks.key, tkey, ks.idx, tidx, n, 0, r.bits, s));
+    void *temp;
+    TRY(d.get((char **)&temp, (int64_t)tb));
+    CK(cub::DeviceRadixSort::SortPairs(temp, tb, ks.key, tkey, ks.idx, tidx, n, 0, r.bits, s));
+    r.tkey = tkey;
+    r.tidx = tidx;
+    k_run_splits<<<(unsigned)(tiles / 256 + 1), 256, 0, s>>>(r, tiles, split);
+    k_merge_runs<<<(unsigned)tiles, kRunThreads, 0, s>>>(r, ev, nv, split, d_ptr, otail, ow, oaos);
+    *launches += 2;
+    CK(cudaGetLastError());
+  }
+  CK(cudaStreamSynchronize(s));
+  return GLV_OK;
+}
+
 // Device-to-host copy of a large result into ordinary (pageable, possibly
 // never touched) host memory, such as the malloc'd arrays the reference's API
 // returns.  A plain cudaMemcpy into such memory runs at the speed of one
@@ -618,12 +941,21 @@ int glv_build_csr(long NV, long NE, const glv_edge *edges, int flags, glv_graph 
   int64_t *dptr, *order = nullptr, nk = NE;
   TRY(upload_edges(c.s, edges, NE, d, &din));
   TRY(d.get(&dptr, NV + 1));
-  if (NE > 0 && (flags & GLV_CSR_REMOVE_EDGES))
+  const bool merge = merges_rows(flags, NE);
+  KeptSorted ks;
+  if (merge) {
+    TRY(kept_sorted(c.s, NV, NE, aos_view(din), d, &ks, &c.launches));
+    nk = ks.nge;
+  } else if (NE > 0 && (flags & GLV_CSR_REMOVE_EDGES)) {
     TRY(kept_order(c.s, NV, NE, aos_view(din), d, &order, &nk, &c.launches));
+  }
   const int64_t m = 2 * nk;
   TRY(d.get(&dout, m));
-  TRY(row_entries(c.s, NV, nk, order, aos_view(din), (flags & GLV_CSR_SORT_ROWS) != 0, d, dptr,
-                  nullptr, nullptr, dout, &c.launches));
+  if (merge)
+    TRY(merged_rows(c.s, NV, ks, aos_view(din), d, dptr, nullptr, nullptr, dout, &c.launches));
+  else
+    TRY(row_entries(c.s, NV, nk, order, aos_view(din), (flags & GLV_CSR_SORT_ROWS) != 0, d, dptr,
+                    nullptr, nullptr, dout, &c.launches));
   long *hp = (long *)malloc((NV + 1) * sizeof(long));
   glv_edge *he = (glv_edge *)malloc(std::max<int64_t>(m, 1) * sizeof(glv_edge));
   if (!hp || !he) {
@@ -663,11 +995,23 @@ int glv_dev_build_csr(long NV, long NE, const long *d_head, const long *d_tail,
                     reinterpret_cast<const int64_t *>(d_tail), d_weight, 1};
   {
     DevScratch d(s);
-    if (NE > 0 && (flags & GLV_CSR_REMOVE_EDGES))
-      TRY(kept_order(s, NV, NE, ev, d, &order, &nk, &launches));
-    TRY(row_entries(s, NV, nk, order, ev, (flags & GLV_CSR_SORT_ROWS) != 0, d,
-                    reinterpret_cast<int64_t *>(d_ptr), d_tail_out, d_weight_out, nullptr,
-                    &launches));
+    // the merge reads the weights while it writes: not in place
+    const bool in_place = overlap(d_weight, NE * 8, d_ptr, (NV + 1) * 8) ||
+                          overlap(d_weight, NE * 8, d_tail_out, 2 * NE * 4) ||
+                          overlap(d_weight, NE * 8, d_weight_out, 2 * NE * 8);
+    if (merges_rows(flags, NE) && !in_place) {
+      KeptSorted ks;
+      TRY(kept_sorted(s, NV, NE, ev, d, &ks, &launches));
+      nk = ks.nge;
+      TRY(merged_rows(s, NV, ks, ev, d, reinterpret_cast<int64_t *>(d_ptr), d_tail_out,
+                      d_weight_out, nullptr, &launches));
+    } else {
+      if (NE > 0 && (flags & GLV_CSR_REMOVE_EDGES))
+        TRY(kept_order(s, NV, NE, ev, d, &order, &nk, &launches));
+      TRY(row_entries(s, NV, nk, order, ev, (flags & GLV_CSR_SORT_ROWS) != 0, d,
+                      reinterpret_cast<int64_t *>(d_ptr), d_tail_out, d_weight_out, nullptr,
+                      &launches));
+    }
   }
   CK(cudaStreamSynchronize(s));
   g_launches += launches;
