@@ -2125,6 +2125,22 @@ int Engine::cluster_grid(int cl) {
   return cluster_grid_[cl];
 }
 
+// Whether a sweep takes one block per SM instead of as many as fit: a grid
+// barrier over half the blocks is shorter, and steps that give each warp at most
+// one item have no use for the rest (1,200 vertices: a whole run 3.33 -> 3.16 ms,
+// 64 or 8 blocks the same; a planted partition of 100k, whose first levels are
+// past the line, 20.9 either way).  Rows for teams, blocks and hubs keep the full
+// grid: with them on half of it R-MAT 18 took 1 % longer.
+static bool few_rows(const std::vector<StepDesc> &steps, int64_t nsm) {
+  for (const StepDesc &d : steps) {
+    int64_t warps = d.seg[BIN_WARP + 1] - d.seg[BIN_WARP];
+    for (int b = BIN_G4; b < BIN_WARP; ++b)  // 4 to 32 lanes a row
+      warps += (((int64_t)(d.seg[b + 1] - d.seg[b]) << (b + 2)) + 31) / 32;
+    if (d.seg[NBINS] > d.seg[BIN_T128] || warps > 16 * nsm) return false;
+  }
+  return true;
+}
+
 // One cooperative launch per iteration (persist.cuh).  Colour phases: C is
 // updated in place and Q is taken after the sweep; Jacobi phases: targets go
 // to Ctgt, Q is taken on the state before the moves, and the loop rotates
@@ -2297,7 +2313,9 @@ int Engine::run_persistent(const Level &L, const std::vector<ClassSched> &sched,
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_iteration<false>, kPersistThreads,
                                                    kPersistSmem));
   if (per_sm < 1) return fail(GLV_ERR_CUDA, "persistent sweep kernel does not fit on an SM");
-  const int grid = cl > 0 ? cluster_grid(cl) : per_sm * nsm_;
+  int grid = cl > 0 ? cluster_grid(cl) : per_sm * nsm_;
+  if (cl == 0 && merge_tiles(L.nv, L.nnz) <= nsm_ && few_rows(steps, nsm_))
+    grid = std::min(grid, nsm_);
   if (grid < 1) return fail(GLV_ERR_CUDA, "no cluster of the persistent sweep kernel fits");
   double *exx_buf = nullptr;
   if (carry_exx) {
