@@ -326,7 +326,7 @@ static int sorted_pairs(cudaStream_t s, int64_t m, int bits, uint64_t *keys, Dev
   return GLV_OK;
 }
 
-// Whether the pairs are counted by community, on the side with more ids.  Not
+// Whether the pairs are counted by a side's nC communities.  Not
 // with less than two vertices an id (singletons, ids with gaps), where both ways
 // take the same time and this one the memory of an offset per id; not where a
 // community is too large for a block even on average; and below 2^30 vertices,
@@ -418,7 +418,10 @@ static int compare_device(cudaStream_t s, int64_t n, int64_t *dC1, int64_t *dC2,
   CK(cudaMemsetAsync(h1, 0, nC1 * sizeof(*h1), s));
   CK(cudaMemsetAsync(h2, 0, nC2 * sizeof(*h2), s));
   CK(cudaMemsetAsync(acc, 0, 9 * sizeof(*acc), s));
-  const bool by2 = nC2 > nC1, grouped = counts_by_community(n, by2 ? nC2 : nC1);
+  // the side with more ids has the smaller communities; a -1 in C2 becomes id n +
+  // 1, and then C1's ids may still be dense
+  const bool ok1 = counts_by_community(n, nC1), ok2 = counts_by_community(n, nC2);
+  const bool grouped = ok1 || ok2, by2 = ok2 && (nC2 > nC1 || !ok1);
   uint64_t *keys = nullptr;
   int32_t *rank = nullptr;
   if (grouped) TRY(d.get(&rank, n)); else TRY(d.get(&keys, n));

@@ -47,7 +47,7 @@ def test_labels_with_gaps_and_minus_one(oracle, n):
     """Ids with large gaps (more ids than vertices: counted by sorted keys),
     and -1 entries on both sides."""
     rng = np.random.default_rng(n)
-    for top in (3, 10 * n + 7):
+    for top in (3, n // 20 + 2, 10 * n + 7):
         C1, C2 = rng.integers(0, top, n), rng.integers(0, top, n)
         C1[rng.random(n) < 0.1] = -1
         C2[rng.random(n) < 0.1] = -1
