@@ -398,6 +398,17 @@ static int compare_device(cudaStream_t s, int64_t n, int64_t *dC1, int64_t *dC2,
   CK(cudaMemcpyAsync(hfl, fl, sizeof(hfl), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   if ((hfl[0] | hfl[1]) & 4) return fail(GLV_ERR_ARG, "a community id below -1");
+  // The -1 entries of the two sides get different values, and the labels are read
+  // again after that: arrays that share memory (a labelling against itself) are
+  // compared in copies.  Without -1 entries nothing is written.
+  int64_t *const home1 = dC1, *const home2 = dC2;
+  const bool copies = ((hfl[0] | hfl[1]) & 2) && overlap(dC1, n * 8, dC2, n * 8);
+  if (copies) {
+    TRY(d.get(&dC1, n));
+    TRY(d.get(&dC2, n));
+    CK(cudaMemcpyAsync(dC1, home1, n * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
+    CK(cudaMemcpyAsync(dC2, home2, n * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
+  }
   // C1 (:63-87): nC1 = largest id, plus one when 0 is an id; -1 entries
   // become nC1, which then grows by one
   const bool z1 = hfl[0] & 1, z2 = hfl[1] & 1;
@@ -427,6 +438,10 @@ static int compare_device(cudaStream_t s, int64_t n, int64_t *dC1, int64_t *dC2,
   if (grouped) TRY(d.get(&rank, n)); else TRY(d.get(&keys, n));
   k_label_pairs<<<csr_grid(n), 256, 0, s>>>(n, dC1, dC2, fill1, n + 1, base1, base2, bits2, h1,
                                             h2, keys, rank, by2);
+  if (copies) {  // C2's values last, as each entry's two stores stand
+    CK(cudaMemcpyAsync(home1, dC1, n * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
+    CK(cudaMemcpyAsync(home2, dC2, n * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
+  }
   k_pair_sum<<<csr_grid(nC1), 256, 0, s>>>(nC1, h1, acc + 1);
   k_pair_sum<<<csr_grid(nC2), 256, 0, s>>>(nC2, h2, acc + 2);
   *launches += 3;
