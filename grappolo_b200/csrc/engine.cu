@@ -4164,20 +4164,21 @@ __global__ void __launch_bounds__(256) k_modularity_static(int64_t nv, const int
   __shared__ MergeSmem sm;
   __shared__ double sh[8];
   __shared__ int s_hit;
-  const int64_t nnz = ptr[nv], ntiles = merge_tiles(nv, nnz);
+  // the rows may be a stretch of a longer CSR: entries p0 to ptr[nv]
+  const int64_t p0 = ptr[0], nnz = ptr[nv] - p0, ntiles = merge_tiles(nv, nnz);
   const int64_t tb = ntiles * blockIdx.x / gridDim.x, te = ntiles * (blockIdx.x + 1) / gridDim.x;
   double ex = 0.0, a2 = 0.0;
   int64_t i0 = 0;
   if (te > tb) {
     const int64_t d = tb * (int64_t)kMergeTile;
-    i0 = block_split(ptr, d, max((int64_t)0, d - nnz), min(d, nv), &s_hit);
+    i0 = block_split(ptr, d + p0, max((int64_t)0, d - nnz), min(d, nv), &s_hit);
   }
   for (int64_t tile = tb; tile < te; ++tile) {
     const int64_t d0 = tile * (int64_t)kMergeTile;
     const int64_t d1 = min(d0 + (int64_t)kMergeTile, nv + nnz);
     const int64_t i1 =
-        block_split(ptr, d1, max(i0, d1 - nnz), min(i0 + (d1 - d0), nv), &s_hit);
-    const int64_t j0 = d0 - i0, j1 = d1 - i1;
+        block_split(ptr, d1 + p0, max(i0, d1 - nnz), min(i0 + (d1 - d0), nv), &s_hit);
+    const int64_t j0 = p0 + d0 - i0, j1 = p0 + d1 - i1;
     for (int64_t i = i0 + threadIdx.x; i < i1; i += 256) {
       const double dg = cDeg[i];
       a2 = __dadd_rn(a2, __dmul_rn(dg, dg));
