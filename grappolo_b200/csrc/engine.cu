@@ -4114,16 +4114,15 @@ int glv_decide_batch(long nv, const long *ptr, const long *tail, const double *w
 
 namespace glv {
 
-// Largest vertex count the static scratch covers: one partial pair per 256
-// vertices, 65,536 pairs -> 16,777,216 vertices, 1 MiB of device memory that
-// every GPU which loads this library keeps until the process exits.
-constexpr int64_t kStaticModParts = 65536;
-constexpr int64_t kStaticModMaxVertices = 16777216;  // the documented limit of the entry
-constexpr int64_t kStaticModBlocks = 148 * 4;
+// The entry's vertex limit belongs to its interface; the scratch does not grow
+// with the graph.
+constexpr int64_t kStaticModMaxVertices = 16777216;
+constexpr int64_t kStaticModBlocks = 148 * 4;  // most blocks of k_modularity_static
 
-// Block partials of e_xx (first half) and a2_x (second half).  Shared by every
+// Block partials of e_xx (first half) and a2_x (second half), 9.5 kB that every
+// GPU which loads this library keeps until the process exits.  Shared by every
 // call on a device: concurrent calls on that device race on it.
-static __device__ __align__(256) double g_mod_scratch[2 * kStaticModParts];
+static __device__ __align__(256) double g_mod_scratch[2 * kStaticModBlocks];
 
 static std::mutex g_mod_scratch_mu;
 static double *g_mod_scratch_addr[kMaxDevices];  // device address of g_mod_scratch, per device
@@ -4229,8 +4228,8 @@ extern "C" int glv_dev_modularity_static(long nv, const long *d_ptr, const int *
   if (nv < 1) return fail(GLV_ERR_ARG, "glv_dev_modularity_static: numVertices < 1");
   if (nv > kStaticModMaxVertices)
     return fail(GLV_ERR_LIMIT,
-                "glv_dev_modularity_static: numVertices exceeds 16,777,216, the size its "
-                "static scratch covers; use the allocating entry points");
+                "glv_dev_modularity_static: numVertices exceeds 16,777,216; use the "
+                "allocating entry points");
   if (!d_ptr || !d_tail || !d_weight || !d_C || !d_cDeg || !d_out)
     return fail(GLV_ERR_ARG, "glv_dev_modularity_static: NULL pointer");
   int ndev = 0;
@@ -4261,7 +4260,7 @@ extern "C" int glv_dev_modularity_static(long nv, const long *d_ptr, const int *
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // four blocks per SM, fewer where the vertices do not give each 32 rows
   const int nparts = (int)std::max<int64_t>(8, std::min<int64_t>(nv / 32, kStaticModBlocks));
-  double *part_e = scratch, *part_a = scratch + kStaticModParts;
+  double *part_e = scratch, *part_a = scratch + kStaticModBlocks;
   // Every partial read below is written first by this call's
   // k_modularity_static, so nothing in the scratch needs clearing.
   k_modularity_static<<<nparts, 256, 0, s>>>(nv, (const int64_t *)d_ptr, d_tail, d_weight, d_C,

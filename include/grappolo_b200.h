@@ -379,10 +379,11 @@ int glv_decide_batch(long nv, const long *ptr, const long *tail, const double *w
  * receives {Q, e_xx, a2_x}: e_xx is the sum of w over entries (i, t) with
  * C[t] == C[i] >= 0, a2_x the sum of d_cDeg[c]^2 over all ids c < nv, and
  * Q = e_xx*constant - a2_x*constant^2.
- * Scratch is a 1 MiB static device array compiled into the library, which
- * bounds nv to 16,777,216 (larger nv returns GLV_ERR_LIMIT without touching the
- * GPU).  Every GPU that loads the library holds that array until the process
- * exits.  The first call on a device looks up the array's address (once per
+ * nv is limited to 16,777,216 (larger nv returns GLV_ERR_LIMIT without touching
+ * the GPU).  The rows may be a stretch of a longer CSR: entries d_ptr[0] to
+ * d_ptr[nv] of d_tail and d_weight.  Scratch is a static device array of a few
+ * kB compiled into the library; every GPU that loads the library holds it until
+ * the process exits.  The first call on a device looks up the array's address (once per
  * device, with that device current); make that first call before any stream
  * capture.  The address is kept for the life of the process: after a
  * cudaDeviceReset of that device the entry must not be called again.
