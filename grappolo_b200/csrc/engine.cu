@@ -571,6 +571,9 @@ class Engine {
 };
 
 constexpr int kGroupLower = 2047;    // group_classes' lower row limit
+// Entries of a run's first level from which that limit is tried.  Not the tuner's
+// limit (tune_min_entries): merged steps change decisions, tuning does not.
+constexpr int64_t kGroupLowerMin = int64_t(1) << 24;
 constexpr int kConstParts = 1024;  // blocks of the constant's reduction
 
 static int grid_for(int64_t n, int block, int cap) {
@@ -1678,7 +1681,7 @@ int Engine::coloring_phase(const Level &L, int ncolors, bool stale, double lower
     sweep_rows_ = false;
     return rc;
   };
-  if (phase_index_ == 0 && !bt_ && persistent() && L.nnz >= tune_min_entries()) group_lower_ = -1;
+  if (phase_index_ == 0 && !bt_ && persistent() && L.nnz >= kGroupLowerMin) group_lower_ = -1;
   TRY(make_sched(&sched));
   if (debug) { cudaStreamSynchronize(s_); fprintf(stderr, "grappolo_b200: schedule %.4f s\n", now_s() - td); }
   dfree(d_sub);
