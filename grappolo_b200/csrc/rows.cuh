@@ -253,15 +253,16 @@ __device__ __forceinline__ void small_decide(const SweepArgs &a, int pos, const 
   double sum, own_w = 0.0, self_w = 0.0;  // Counter[c], Counter[own], self-loops
   bool cand;                              // this lane offers community c
   if (G <= 8) {
-    // every lane sees the other lanes of its row in turn (3 shuffles each; a
-    // match over the warp takes up to 379 cycles); the top bit marks self-loops
+    // every lane sees all entries of its row in order (3 shuffles each; a match
+    // over the warp takes up to 379 cycles); the top bit marks self-loops.  In
+    // order, so that every lane of the row has the same sums on any weights:
+    // from each lane's own entry on, candidates of equal gain differed in the
+    // last bit.
     const int32_t mark = (has && t == r.v) ? (c | INT32_MIN) : (has ? c : 0x7fffffff);
-    sum = has ? w : 0.0;
-    if (c == own && has) own_w = w;
-    if (has && t == r.v) self_w = w;
+    sum = 0.0;
 #pragma unroll
-    for (int off = 1; off < G; ++off) {
-      const int src = (lane & ~(G - 1)) | ((gl + off) & (G - 1));
+    for (int q = 0; q < G; ++q) {
+      const int src = (lane & ~(G - 1)) | q;
       const int32_t oc = __shfl_sync(FULL, mark, src);
       const double ow = __shfl_sync(FULL, w, src);
       const int32_t id = oc & 0x7fffffff;
