@@ -156,11 +156,15 @@ __device__ __forceinline__ int group_slots(int size) {
 }
 
 // Communities of up to kGroupWarp vertices, one per warp; larger ones are
-// listed: nlist[0] for blocks, nlist[1] for sorting (their vertices in total[0]).
+// listed: *nblock for blocks; for sorting with the vertices listed before, and
+// *total counts both the communities (from kSortCount up) and their vertices.
+constexpr int kSortShift = 34;  // vertices stay below 2^30
+constexpr unsigned long long kSortCount = 1ull << kSortShift;
+
 __global__ void __launch_bounds__(256) k_group_pairs_warp(
     int64_t nC, const unsigned long long *size, const int64_t *off, const int32_t *other,
-    unsigned long long *out, int32_t *list_block, int32_t *list_sort, int32_t *nlist,
-    unsigned long long *total) {
+    unsigned long long *out, int32_t *list_block, int32_t *list_sort, int32_t *sort_start,
+    int32_t *nblock, unsigned long long *total) {
   __shared__ int32_t s_key[8][512];
   __shared__ uint32_t s_cnt[8][512];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -173,10 +177,11 @@ __global__ void __launch_bounds__(256) k_group_pairs_warp(
     if (n > kGroupWarp) {
       if (lane == 0) {
         if (n <= kGroupBlock) {
-          list_block[atomicAdd(&nlist[0], 1)] = (int32_t)c;
+          list_block[atomicAdd(nblock, 1)] = (int32_t)c;
         } else {
-          list_sort[atomicAdd(&nlist[1], 1)] = (int32_t)c;
-          atomicAdd(total, n);
+          const unsigned long long at = atomicAdd(total, kSortCount | n);
+          list_sort[at >> kSortShift] = (int32_t)c;
+          sort_start[at >> kSortShift] = (int32_t)(at & (kSortCount - 1));
         }
       }
       continue;
@@ -199,10 +204,10 @@ __global__ void __launch_bounds__(256) k_group_pairs_warp(
 // The listed communities of up to kGroupBlock vertices, one per block.
 __global__ void __launch_bounds__(512) k_group_pairs_block(
     const unsigned long long *size, const int64_t *off, const int32_t *other,
-    const int32_t *list, const int32_t *nlist, unsigned long long *out) {
+    const int32_t *list, const int32_t *nblock, unsigned long long *out) {
   extern __shared__ int32_t s_table[];
   unsigned long long acc = 0;
-  const int lane = threadIdx.x & 31, nl = nlist[0];
+  const int lane = threadIdx.x & 31, nl = *nblock;
   for (int t = blockIdx.x; t < nl; t += gridDim.x) {
     const int32_t c = list[t];
     const int m = (int)size[c], slots = group_slots(m);
@@ -222,26 +227,28 @@ __global__ void __launch_bounds__(512) k_group_pairs_block(
   if (lane == 0 && acc) atomicAdd(out, acc);
 }
 
-// The keys (community above label) of the communities listed for sorting;
-// placed[0] hands out places.
+// The keys (community above label) of the nl communities listed for sorting, of
+// `left` vertices: a block takes 8192 places of the whole list, which are at most
+// three communities.  (All blocks over each community in turn left one or two
+// of them busy: 20M vertices in communities of 3000 to 9000 13.9 ms, now 1.25.)
 __global__ void __launch_bounds__(512) k_group_keys(const unsigned long long *size,
                                                     const int64_t *off, const int32_t *other,
-                                                    const int32_t *list, const int32_t *nlist,
-                                                    int bits, unsigned long long *placed,
+                                                    const int32_t *list, const int32_t *start,
+                                                    int nl, int64_t left, int bits,
                                                     uint64_t *keys) {
-  __shared__ unsigned long long s_at;
-  const int nl = nlist[1];
-  for (int t = 0; t < nl; ++t) {
-    // all blocks share each community: chunks of 8192 labels
-    const int32_t c = list[t];
-    const int64_t m = (int64_t)size[c];
-    for (int64_t k0 = (int64_t)blockIdx.x * 8192; k0 < m; k0 += (int64_t)gridDim.x * 8192) {
-      const int64_t k1 = min(m, k0 + 8192);
-      __syncthreads();
-      if (threadIdx.x == 0) s_at = atomicAdd(placed, (unsigned long long)(k1 - k0));
-      __syncthreads();
-      for (int64_t k = k0 + threadIdx.x; k < k1; k += 512)
-        keys[s_at + (k - k0)] = ((uint64_t)c << bits) | (uint32_t)other[off[c] + k];
+  for (int64_t p0 = (int64_t)blockIdx.x * 8192; p0 < left; p0 += (int64_t)gridDim.x * 8192) {
+    const int64_t p1 = min(left, p0 + 8192);
+    int lo = 0, hi = nl - 1;  // the community that holds place p0
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (start[mid] <= p0) lo = mid; else hi = mid - 1;
+    }
+    for (int t = lo; t < nl && start[t] < p1; ++t) {
+      const int32_t c = list[t];
+      const int64_t b = start[t], e = b + (int64_t)size[c];
+      const int32_t *lab = other + off[c];
+      for (int64_t p = max(b, p0) + threadIdx.x; p < min(e, p1); p += 512)
+        keys[p] = ((uint64_t)c << bits) | (uint32_t)lab[p - b];
     }
   }
 }
@@ -333,7 +340,7 @@ static int sorted_pairs(cudaStream_t s, int64_t m, int bits, uint64_t *keys, Dev
 // so that sorting every community after all still fits the scratch that
 // sorting all keys takes at 2^31.  20M vertices, 20 % noise: communities of 20 1.91
 // -> 1.09 ms, of 150 1.93 -> 0.70, of 5000 1.95 -> 0.75; skewed sizes (k-th label
-// by u^6, most vertices sorted after all) 4.83 -> 4.82.
+// by u^6, most vertices sorted after all) 4.80 -> 3.21, 3000 to 9000 2.03 -> 1.25.
 static bool counts_by_community(int64_t n, int64_t nC) {
   return n < (int64_t(1) << 30) && nC <= n / 2 && n / nC <= kGroupBlock;
 }
@@ -343,12 +350,13 @@ struct LabelGroups {
   int64_t nC = 0;
   const unsigned long long *size = nullptr;
   int64_t *off = nullptr;
-  int32_t *other = nullptr, *list_block = nullptr, *list_sort = nullptr, *nlist = nullptr;
+  int32_t *other = nullptr, *list_block = nullptr, *nblock = nullptr;
+  int32_t *list_sort = nullptr, *sort_start = nullptr;
 };
 
 // *pairs += sum of C(n_ab, 2) over the communities of up to kGroupBlock vertices of
 // the side with g->nC communities of g->size (labels Cg); rank from
-// k_label_pairs.  total[0] += the vertices of the larger ones.
+// k_label_pairs.  *total counts the larger ones (k_group_pairs_warp).
 static int grouped_pairs(cudaStream_t s, int64_t n, const int64_t *Cg, const int64_t *Co,
                          int64_t baseg, int64_t baseo, const int32_t *rank, DevScratch &d,
                          LabelGroups *g, unsigned long long *pairs, unsigned long long *total,
@@ -358,8 +366,9 @@ static int grouped_pairs(cudaStream_t s, int64_t n, const int64_t *Cg, const int
   TRY(d.get(&g->other, n));
   TRY(d.get(&g->list_block, most_block));
   TRY(d.get(&g->list_sort, n / (kGroupBlock + 1) + 1));
-  TRY(d.get(&g->nlist, 2));
-  CK(cudaMemsetAsync(g->nlist, 0, 2 * sizeof(int32_t), s));
+  TRY(d.get(&g->sort_start, n / (kGroupBlock + 1) + 1));
+  TRY(d.get(&g->nblock, 1));
+  CK(cudaMemsetAsync(g->nblock, 0, sizeof(int32_t), s));
   const int64_t *size = reinterpret_cast<const int64_t *>(g->size);
   size_t tb = 0;
   CK(cub::DeviceScan::ExclusiveSum(nullptr, tb, size, g->off, g->nC, s));
@@ -368,11 +377,12 @@ static int grouped_pairs(cudaStream_t s, int64_t n, const int64_t *Cg, const int
   CK(cub::DeviceScan::ExclusiveSum(temp, tb, size, g->off, g->nC, s));
   k_group_labels<<<csr_grid(n), 256, 0, s>>>(n, Cg, Co, baseg, baseo, g->off, rank, g->other);
   k_group_pairs_warp<<<(unsigned)std::min<int64_t>((g->nC + 7) / 8, 148 * 6), 256, 0, s>>>(
-      g->nC, g->size, g->off, g->other, pairs, g->list_block, g->list_sort, g->nlist, total);
+      g->nC, g->size, g->off, g->other, pairs, g->list_block, g->list_sort, g->sort_start,
+      g->nblock, total);
   const int smem = 8192 * 8;
   CK(cudaFuncSetAttribute(k_group_pairs_block, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   k_group_pairs_block<<<(unsigned)std::min<int64_t>(most_block, 148 * 3), 512, smem, s>>>(
-      g->size, g->off, g->other, g->list_block, g->nlist, pairs);
+      g->size, g->off, g->other, g->list_block, g->nblock, pairs);
   *launches += 3;
   CK(cudaGetLastError());
   return GLV_OK;
@@ -425,10 +435,10 @@ static int compare_device(cudaStream_t s, int64_t n, int64_t *dC1, int64_t *dC2,
   unsigned long long *h1, *h2, *acc;
   TRY(d.get(&h1, nC1));
   TRY(d.get(&h2, nC2));
-  TRY(d.get(&acc, 9));  // pairs, pairs of C1, of C2, Gini sums of both, vertices left to sort, placed
+  TRY(d.get(&acc, 8));  // pairs, pairs of C1, of C2, Gini sums of both, left to sort
   CK(cudaMemsetAsync(h1, 0, nC1 * sizeof(*h1), s));
   CK(cudaMemsetAsync(h2, 0, nC2 * sizeof(*h2), s));
-  CK(cudaMemsetAsync(acc, 0, 9 * sizeof(*acc), s));
+  CK(cudaMemsetAsync(acc, 0, 8 * sizeof(*acc), s));
   // the side with more ids has the smaller communities; a -1 in C2 becomes id n +
   // 1, and then C1's ids may still be dense
   const bool ok1 = counts_by_community(n, nC1), ok2 = counts_by_community(n, nC2);
@@ -446,7 +456,7 @@ static int compare_device(cudaStream_t s, int64_t n, int64_t *dC1, int64_t *dC2,
   k_pair_sum<<<csr_grid(nC2), 256, 0, s>>>(nC2, h2, acc + 2);
   *launches += 3;
   CK(cudaGetLastError());
-  unsigned long long *srt, pairs[9];
+  unsigned long long *srt, pairs[8];
   // community sizes are at most n: sort only the bits that can be set
   const int size_bits = id_bits(n + 1);
   TRY(gini_sums(s, h1, nC1, size_bits, d, &srt, acc + 3, launches));
@@ -463,10 +473,11 @@ static int compare_device(cudaStream_t s, int64_t n, int64_t *dC1, int64_t *dC2,
   CK(cudaMemcpyAsync(pairs, acc, sizeof(pairs), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   if (pairs[7] > 0) {
-    const int64_t left = (int64_t)pairs[7];
+    const int64_t left = (int64_t)(pairs[7] & (kSortCount - 1));
     TRY(d.get(&keys, left));
     k_group_keys<<<(unsigned)std::min<int64_t>((left + 8191) / 8192, 148 * 4), 512, 0, s>>>(
-        g.size, g.off, g.other, g.list_sort, g.nlist, by2 ? bits1 : bits2, acc + 8, keys);
+        g.size, g.off, g.other, g.list_sort, g.sort_start, (int)(pairs[7] >> kSortShift), left,
+        by2 ? bits1 : bits2, keys);
     ++*launches;
     CK(cudaGetLastError());
     TRY(sorted_pairs(s, left, bits1 + bits2, keys, d, acc, launches));
