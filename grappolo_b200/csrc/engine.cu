@@ -4158,29 +4158,28 @@ __device__ __forceinline__ int64_t block_split(const int64_t *ptr, int64_t d, in
 // vertices each took 6.65 ms on R-MAT 22 (123M entries), as long as the block
 // that holds the hubs; equal tiles take 0.91 ms
 // (12 B per entry and 16 B per vertex: 1.5 GB, 0.24 ms at the measured copy rate;
-// the 123M gathers of C move 3.9 GB of L2 sectors).
-__global__ void __launch_bounds__(256) k_modularity_static(int64_t nv, const int64_t *ptr,
-                                                           const int32_t *tail, const double *w,
-                                                           const int32_t *C, const double *cDeg,
-                                                           double *part_e, double *part_a) {
+// the 123M gathers of C move 3.9 GB of L2 sectors).  Four blocks per SM, as the
+// grid has them: with 80 registers three fit, and the fourth's tiles came after
+// the others' (1.21 ms).
+__global__ void __launch_bounds__(256, 4)
+    k_modularity_static(int64_t nv, const int64_t *ptr, const int32_t *tail, const double *w,
+                        const int32_t *C, const double *cDeg, double *part_e, double *part_a) {
   __shared__ MergeSmem sm;
   __shared__ double sh[8];
   __shared__ int s_hit;
-  // the rows may be a stretch of a longer CSR: entries p0 to ptr[nv]
-  const int64_t p0 = ptr[0], nnz = ptr[nv] - p0, ntiles = merge_tiles(nv, nnz);
+  // the rows may be a stretch of a longer CSR: its entries, and the items of the
+  // merge sequence, are counted from ptr[0] on
+  const int64_t end = ptr[nv], first = ptr[0], ntiles = merge_tiles(nv, end - first);
   const int64_t tb = ntiles * blockIdx.x / gridDim.x, te = ntiles * (blockIdx.x + 1) / gridDim.x;
+  const int64_t db = first + tb * (int64_t)kMergeTile, de = first + te * (int64_t)kMergeTile;
   double ex = 0.0, a2 = 0.0;
   int64_t i0 = 0;
-  if (te > tb) {
-    const int64_t d = tb * (int64_t)kMergeTile;
-    i0 = block_split(ptr, d + p0, max((int64_t)0, d - nnz), min(d, nv), &s_hit);
-  }
-  for (int64_t tile = tb; tile < te; ++tile) {
-    const int64_t d0 = tile * (int64_t)kMergeTile;
-    const int64_t d1 = min(d0 + (int64_t)kMergeTile, nv + nnz);
+  if (te > tb) i0 = block_split(ptr, db, max((int64_t)0, db - end), min(db - first, nv), &s_hit);
+  for (int64_t d0 = db; d0 < de; d0 += kMergeTile) {
+    const int64_t d1 = min(d0 + (int64_t)kMergeTile, nv + end);
     const int64_t i1 =
-        block_split(ptr, d1 + p0, max(i0, d1 - nnz), min(i0 + (d1 - d0), nv), &s_hit);
-    const int64_t j0 = p0 + d0 - i0, j1 = p0 + d1 - i1;
+        block_split(ptr, d1, max(i0, d1 - end), min(i0 + (d1 - d0), nv), &s_hit);
+    const int64_t j0 = d0 - i0, j1 = d1 - i1;
     for (int64_t i = i0 + threadIdx.x; i < i1; i += 256) {
       const double dg = cDeg[i];
       a2 = __dadd_rn(a2, __dmul_rn(dg, dg));
