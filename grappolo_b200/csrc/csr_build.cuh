@@ -377,13 +377,29 @@ static int row_entries(cudaStream_t s, int64_t nv, int64_t nk, const int64_t *or
 //
 // Equal entries come latest first, by the slots removeEdges leaves the edges in:
 // an edge below NGE keeps its slot, and the q-th kept edge from NGE on fills the
-// q-th hole from the end.  Only ties need slots, so only the dropped places are
-// kept, in order: the holes are those below NGE.
+// q-th hole from the end.  Only ties need slots; they come from a bitmap of the
+// dropped places with the count before every 128 (two loads a count, both from
+// L2), and the holes, the dropped places below NGE, in order.  (A sorted list of
+// all dropped places, searched for every tie, cost more than it saved where most
+// edges are repeats: 20M edges over 1000 vertices 1.39 ms by sorting all entries,
+// 1.59 that way, 1.07 this way.)
+constexpr int kDropBlock = 128;  // places to a count
 struct KeptSorted {
   int64_t nge = 0, ndrop = 0;
-  uint64_t *key = nullptr;   // kept edges by (head, tail): head << bits | tail
-  int32_t *idx = nullptr;    // their places in the list
-  int32_t *drop = nullptr;   // dropped places, ascending
+  uint64_t *key = nullptr;    // kept edges by (head, tail): head << bits | tail
+  int32_t *idx = nullptr;     // their places in the list
+  uint32_t *dropped = nullptr;  // bitmap over the list
+  int32_t *before = nullptr;  // dropped places before each kDropBlock
+  int32_t *hole = nullptr;    // the holes, ascending
+};
+
+__device__ __forceinline__ int drop_count(const uint4 &w) {
+  return __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
+}
+
+struct DropCount {  // dropped places of each kDropBlock
+  const uint4 *words;
+  __device__ int32_t operator()(int32_t b) const { return drop_count(words[b]); }
 };
 
 constexpr int kPickItems = 8;            // records a lane of k_pick
@@ -411,16 +427,16 @@ __device__ __forceinline__ bool run_first(const uint64_t *skeys, int64_t s, int 
   return (k >> bits) != (k & ((1ull << bits) - 1)) && (s == 0 || skeys[s - 1] != k);
 }
 
-// One block per tile of sorted records.  idx null: kept[tile] = its kept
+// One block per tile of sorted records.  Not kWrite: kept[tile] = its kept
 // records; otherwise they go to key / idx from kept[tile] (the tile's offset)
-// on, in order, and the other records' places to drop.  A warp takes 256
+// on, in order, and the other records' places are set in dropped.  A warp takes 256
 // records in a row, so its writes are coalesced (two passes over the keys,
 // 8 + 24 bytes a record, 0.58 ms for 67M; a scatter of one flag byte per record
 // to its place in the list and selections from those flags took 1.3).
 template <bool kWrite>
 __global__ void __launch_bounds__(256) k_pick(int64_t ne, int bits, const uint64_t *skeys,
                                               const int32_t *sidx, int64_t *kept, uint64_t *key,
-                                              int32_t *idx, int32_t *drop) {
+                                              int32_t *idx, uint32_t *dropped) {
   __shared__ int s_n[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t s0 = (int64_t)blockIdx.x * kPickTile + warp * (32 * kPickItems);
@@ -455,19 +471,40 @@ __global__ void __launch_bounds__(256) k_pick(int64_t ne, int bits, const uint64
         key[p] = k[u];
         idx[p] = sidx[s];
       } else {
-        drop[s - p] = sidx[s];
+        const int32_t i = sidx[s];
+        atomicOr(&dropped[i >> 5], 1u << (i & 31));
       }
     }
   }
 }
 
-__device__ __forceinline__ int64_t drops_below(const KeptSorted &ks, int64_t place) {
-  int64_t lo = 0, hi = ks.ndrop;
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (ks.drop[mid] < place) lo = mid + 1; else hi = mid;
+// The holes in order; one thread per kDropBlock places.
+__global__ void k_holes(int64_t nge, const uint4 *words, const int32_t *before, int32_t *hole) {
+  const int64_t nb = (nge + kDropBlock - 1) / kDropBlock;
+  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
+       b += (int64_t)gridDim.x * blockDim.x) {
+    const uint4 w = words[b];
+    const uint32_t part[4] = {w.x, w.y, w.z, w.w};
+    int64_t at = before[b];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      for (uint32_t rem = part[q]; rem; rem &= rem - 1) {
+        const int64_t place = b * kDropBlock + 32 * q + __ffs(rem) - 1;
+        if (place < nge) hole[at++] = (int32_t)place;
+      }
   }
-  return lo;
+}
+
+__device__ __forceinline__ int64_t drops_below(const KeptSorted &ks, int64_t place) {
+  const int64_t b = place / kDropBlock;
+  uint4 w = reinterpret_cast<const uint4 *>(ks.dropped)[b];
+  const int q = (int)(place % kDropBlock) >> 5;
+  const uint32_t low = (1u << (place & 31)) - 1u;  // of the word that holds place
+  w.x &= q > 0 ? ~0u : low;
+  w.y &= q > 1 ? ~0u : (q == 1 ? low : 0u);
+  w.z &= q > 2 ? ~0u : (q == 2 ? low : 0u);
+  w.w &= q == 3 ? low : 0u;
+  return ks.before[b] + drop_count(w);
 }
 
 // The slot that removeEdges leaves the kept list edge i in.
@@ -475,7 +512,7 @@ __device__ __forceinline__ int64_t kept_slot(const KeptSorted &ks, int32_t i) {
   if (i < ks.nge) return i;
   const int64_t holes = drops_below(ks, ks.nge);
   const int64_t q = (i - ks.nge) - (drops_below(ks, i) - holes);
-  return ks.drop[holes - 1 - q];
+  return ks.hole[holes - 1 - q];
 }
 
 // The two lists of directed entries: by head as the kept edges stand, by tail
@@ -642,17 +679,23 @@ static int kept_sorted(cudaStream_t s, int64_t nv, int64_t ne, EdgeView ev, DevS
   ks->key = k1;
   ks->idx = v1;
   ks->ndrop = ne - ks->nge;
-  int32_t *drop = nullptr, *order = nullptr;
-  TRY(d.get(&drop, ks->ndrop)); TRY(d.get(&order, ks->ndrop));
-  k_pick<true><<<(unsigned)tiles, 256, 0, s>>>(ne, bits, k2, v2, cnt, k1, v1, drop);
+  const int64_t nb = (ne + kDropBlock - 1) / kDropBlock;
+  TRY(d.get(&ks->dropped, nb * (kDropBlock / 32)));
+  CK(cudaMemsetAsync(ks->dropped, 0, nb * (kDropBlock / 8), s));
+  k_pick<true><<<(unsigned)tiles, 256, 0, s>>>(ne, bits, k2, v2, cnt, k1, v1, ks->dropped);
   CK(cudaGetLastError());
   *launches += 3;
-  ks->drop = order;
   if (ks->ndrop > 0 && ks->nge > 0) {
-    const int pb = id_bits(ne);
-    CK(cub::DeviceRadixSort::SortKeys(nullptr, t2, drop, order, ks->ndrop, 0, pb, s));
+    const uint4 *words = reinterpret_cast<const uint4 *>(ks->dropped);
+    const auto count = thrust::make_transform_iterator(thrust::counting_iterator<int32_t>(0),
+                                                       DropCount{words});
+    TRY(d.get(&ks->before, nb)); TRY(d.get(&ks->hole, std::min(ks->nge, ks->ndrop)));
+    CK(cub::DeviceScan::ExclusiveSum(nullptr, t2, count, ks->before, nb, s));
     TRY(d.get((char **)&temp, (int64_t)t2));
-    CK(cub::DeviceRadixSort::SortKeys(temp, t2, drop, order, ks->ndrop, 0, pb, s));
+    CK(cub::DeviceScan::ExclusiveSum(temp, t2, count, ks->before, nb, s));
+    k_holes<<<csr_grid(nb), 256, 0, s>>>(ks->nge, words, ks->before, ks->hole);
+    ++*launches;
+    CK(cudaGetLastError());
   }
   return GLV_OK;
 }

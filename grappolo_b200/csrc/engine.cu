@@ -19,6 +19,7 @@
 
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 #include "batch_kernels.cuh"
 #include "color_flow.cuh"
