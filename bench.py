@@ -176,8 +176,23 @@ def aggregate(seconds, edges, dist=None, device=None):
 
 
 # --------------------------------------------------------------------- reference arm
+def reference_unavailable():
+    """Why the reference cannot be timed here (no build of it, and no sources to build it
+    from), as the line's value, or None."""
+    from oracle import ReferenceMissing, reference_library
+    try:
+        reference_library(fast=True)
+    except ReferenceMissing as e:
+        return {'unavailable': str(e)}
+    return None
+
+
 def run_reference(args, rank):
     if rank != 0:
+        return 0
+    missing = reference_unavailable()
+    if missing:
+        print(json.dumps({'impl': 'reference', **missing}), flush=True)
         return 0
     if args.workload == 'csr':
         return run_csr_reference(args)
@@ -436,11 +451,13 @@ def run_compare_workload(args, world, rank, local):
         del np
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        cv, cdt, cn, cores = compare_cpu_sample(min(args.scale, 20))
-        cpu = {'value': cv, 'unit': CMP_UNIT, 'cores': cores, 'kind': 'reference',
-               'sample': f'reference computeCommunityComparisons, one thread (its nested '
-                         f'OpenMP regions repeat all work per thread), -Ofast build, on {cn} '
-                         f'vertices ({cdt:.2f} s)'}
+        cpu = reference_unavailable()
+        if cpu is None:
+            cv, cdt, cn, cores = compare_cpu_sample(min(args.scale, 20))
+            cpu = {'value': cv, 'unit': CMP_UNIT, 'cores': cores, 'kind': 'reference',
+                   'sample': f'reference computeCommunityComparisons, one thread (its nested '
+                             f'OpenMP regions repeat all work per thread), -Ofast build, on {cn} '
+                             f'vertices ({cdt:.2f} s)'}
     extra = {'f_score': st['f_score'], 'same_same': st['same_same']}
     line = {'metric': CMP_METRIC, 'value': n_all / t_max, 'unit': CMP_UNIT, 'n_gpus': world,
             'steps': args.steps, 'warmup': args.warmup, 'ms_per_step': 1e3 * t / args.steps,
@@ -546,9 +563,11 @@ def run_csr_workload(args, world, rank, local):
         del aos
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        cv, cdt, cne = csr_cpu_sample(args.csr_sample_scale)
-        cpu = {'value': cv, 'unit': CSR_UNIT, 'cores': 1, 'kind': 'reference',
-               'sample': csr_sample_text(args.csr_sample_scale, cdt, cne)}
+        cpu = reference_unavailable()
+        if cpu is None:
+            cv, cdt, cne = csr_cpu_sample(args.csr_sample_scale)
+            cpu = {'value': cv, 'unit': CSR_UNIT, 'cores': 1, 'kind': 'reference',
+                   'sample': csr_sample_text(args.csr_sample_scale, cdt, cne)}
     line = {'metric': CSR_METRIC, 'value': value, 'unit': CSR_UNIT, 'n_gpus': world,
             'steps': args.steps, 'warmup': args.warmup, 'ms_per_step': 1e3 * t / args.steps,
             'higher_is_better': True, 'scaling': 'weak', 'vs_baseline': None, 'dtype': 'int64',
@@ -646,7 +665,7 @@ def run_batch_workload(args, world, rank, local):
     done, q = per[:, 0], per[:, 1]
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        cpu = batch_cpu_baseline(data[0], args.batch_sample)
+        cpu = reference_unavailable() or batch_cpu_baseline(data[0], args.batch_sample)
     edges = sum(r['edges_swept'] for run in runs for r in run)
     launches = sum(r['kernel_launches'] for run in runs for r in run)
     line = {'metric': 'batched Louvain graphs/s', 'value': g_all / t_max, 'unit': 'graphs/s',
@@ -846,8 +865,8 @@ def main():
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        cpu = cpu_baseline(ptr, tail, w)
-        if args.workload == 'rmat':
+        cpu = reference_unavailable() or cpu_baseline(ptr, tail, w)
+        if args.workload == 'rmat' and 'unavailable' not in cpu:
             cpu['full_run'] = reference_full_run(args.full_run_scale)
 
     peak, peak_kind = measured_peak()

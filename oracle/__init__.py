@@ -5,4 +5,5 @@
 (_ref/libgrappolo_ref.so).  Only tests/, ``__graft_entry__.smoke()`` and the
 CPU-baseline leg of bench.py use them, and only as checkers.
 """
-from .lvoracle import COracle, Reference, PhaseRecord, build  # noqa: F401
+from .lvoracle import (COracle, Reference, ReferenceMissing, PhaseRecord, build,  # noqa: F401
+                       reference_library)

@@ -20,7 +20,7 @@ def build(ref: str | None = None) -> None:
     cmd = ['make', '-s', '-C', HERE, '-j8', 'all']
     if ref:
         cmd.append(f'REF={ref}')
-    subprocess.run(cmd, check=True)
+    subprocess.run(cmd, check=True, stdout=2)  # stdout is the caller's
 
 
 def _lp(a: np.ndarray):
@@ -335,6 +335,24 @@ def parse_comparison_log(text: str) -> dict:
     return out
 
 
+class ReferenceMissing(RuntimeError):
+    """Grappolo's own functions were not built, and its sources are not here to build them."""
+
+
+def reference_library(fast: bool = False, patched_vbase: bool = False) -> str:
+    """Path of a build of Grappolo's own functions, built now if it can be."""
+    name = 'libgrappolo_ref_fast.so' if fast else 'libgrappolo_ref.so'
+    if patched_vbase:
+        name = 'libgrappolo_ref_vbase.so'
+    path = os.path.join(HERE, '_ref', name)
+    if not os.path.exists(path):
+        build()
+    if not os.path.exists(path):
+        raise ReferenceMissing(f'oracle/_ref/{name} is not built, and the reference tree it is '
+                               f'compiled from is absent')
+    return path
+
+
 class Reference:
     """Grappolo's own functions, compiled from its sources (oracle/_ref)."""
 
@@ -342,13 +360,7 @@ class Reference:
         """patched_vbase loads the build whose vBaseRedistribution gains its missing
         return (oracle/ref_vbase.cpp), so coloring = 2 runs; its type 0 is defined
         only where the oracle reports no stuck vertex."""
-        name = 'libgrappolo_ref_fast.so' if fast else 'libgrappolo_ref.so'
-        if patched_vbase:
-            name = 'libgrappolo_ref_vbase.so'
-        path = os.path.join(HERE, '_ref', name)
-        if not os.path.exists(path):
-            build()
-        L = ct.CDLL(path)
+        L = ct.CDLL(reference_library(fast, patched_vbase))
         self.L = L
         L.ref_color.restype = ct.c_int
         L.ref_color_mhash.restype = ct.c_int

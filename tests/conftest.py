@@ -12,6 +12,17 @@ def pytest_configure(config):
     config.addinivalue_line('markers', 'gpu: needs a CUDA device (B200)')
 
 
+@pytest.hookimpl(wrapper=True)
+def pytest_pyfunc_call(pyfuncitem):
+    """A test that loads the reference itself is skipped where it was not built, as the
+    users of the `reference` fixture are."""
+    from oracle import ReferenceMissing
+    try:
+        return (yield)
+    except ReferenceMissing as e:
+        pytest.skip(str(e))
+
+
 @pytest.fixture(scope='session')
 def oracle():
     from oracle import COracle
