@@ -460,6 +460,7 @@ class Engine {
   int hub_offsets(const Level &L, std::vector<ClassSched> &sched, bool tables);
   int group_classes(const Level &L, int ncolors, std::vector<ClassSched> *sched);
   int sublevels(const Level &L, int ncolors, int32_t **d_sub, int *nsub);
+  int launch_short_bin(int b, int64_t lo, int64_t hi, const SweepArgs &a);
   int launch_sweep(const Level &L, const Step &st, SweepArgs a, bool ordered, Probes *pr);
   int launch_apply(const ClassSched &cs, bool ordered);
   int launch_modularity(const Level &L, const int32_t *Cm, const double *ownw);
@@ -1513,31 +1514,65 @@ int Engine::recolor(const Level &L, int *ncolors, int passes) {
 constexpr int kWarpCap = 256;   // table_cap(127)
 constexpr int kBlockCap = 8192; // table_cap(4095)
 
+// The rows of one bin of up to 127 entries, in entry order, on as many warps as
+// the GPU holds.
+int Engine::launch_short_bin(int b, int64_t lo, int64_t hi, const SweepArgs &a) {
+  const int64_t n = hi - lo;
+  const int cap = nsm_ * 16;
+  switch (b) {
+    case BIN_G4:
+      LAUNCH(k_sweep_small<4>, grid_for(n * 4, 256, cap), 256, 0, s_, a, lo, hi);
+      break;
+    case BIN_G8:
+      LAUNCH(k_sweep_small<8>, grid_for(n * 8, 256, cap), 256, 0, s_, a, lo, hi);
+      break;
+    case BIN_G16:
+      LAUNCH(k_sweep_small<16>, grid_for(n * 16, 256, cap), 256, 0, s_, a, lo, hi);
+      break;
+    case BIN_G32:
+      LAUNCH(k_sweep_small<32>, grid_for(n * 32, 256, cap), 256, 0, s_, a, lo, hi);
+      break;
+    case BIN_WARP: {
+      const size_t smem = 8 * kWarpCap * (sizeof(double) + sizeof(int32_t));
+      LAUNCH(k_sweep_warp<kWarpCap>, grid_for(n * 32, 256, cap), 256, smem, s_, a, lo, hi);
+      break;
+    }
+  }
+  return GLV_OK;
+}
+
 int Engine::launch_sweep(const Level &L, const Step &st, SweepArgs a, bool ordered_acc,
                          Probes *pr) {
-  const int cap = nsm_ * 16;
   if (ordered_acc) {
-    // one launch for all bins, or one per bin when each launch is timed
+    // One launch for all bins, or one per bin when each launch is timed.  A bin
+    // with several rows for each of that launch's warps, which the long rows'
+    // tables keep to two blocks per SM, goes alone.
     const bool split = pr && pr->level >= 2;
     for (int first = 0; first < NBINS; ++first) {
       BinRanges r{};
       int64_t nlong = 0, items = 0;
       constexpr int vpw[NBINS] = {8, 4, 2, 1, 1, 0, 0, 0, 0};
+      int pidx = -1;
+      if (pr && (!split || st.seg[first + 1] > st.seg[first]))
+        TRY(pr->begin(first, 2, s_, &pidx));
       for (int b = first; b < (split ? first + 1 : NBINS); ++b) {
+        const int64_t n = st.seg[b + 1] - st.seg[b];
+        const int64_t it = b >= BIN_T128 ? 0 : (n + vpw[b] - 1) / vpw[b];
+        if (it > kOrdOwnItems * kOrdWarps * 2 * nsm_) {
+          TRY(launch_short_bin(b, st.seg[b], st.seg[b + 1], a));
+          continue;
+        }
         r.lo[b] = st.seg[b];
         r.hi[b] = st.seg[b + 1];
-        const int64_t n = r.hi[b] - r.lo[b];
+        items += it;
         if (b >= BIN_T128) nlong += n;
-        else items += (n + vpw[b] - 1) / vpw[b];
       }
       if (nlong + items > 0) {
-        int pidx = -1;
-        if (pr) TRY(pr->begin(first, 2, s_, &pidx));
         const int gl = (int)std::min<int64_t>(nlong, nsm_);
         const int gw = (int)std::min<int64_t>((items + kOrdWarps - 1) / kOrdWarps, nsm_ * 2);
         LAUNCH(k_sweep_ordered, gl + gw, kOrdThreads, kOrdSmem, s_, a, r, gl);
-        if (pr) TRY(pr->end(pidx, s_));
       }
+      if (pidx >= 0) TRY(pr->end(pidx, s_));
       if (!split) break;
     }
     return GLV_OK;
@@ -1549,23 +1584,9 @@ int Engine::launch_sweep(const Level &L, const Step &st, SweepArgs a, bool order
     int pidx = -1;
     if (pr) TRY(pr->begin(b, 2, s_, &pidx));
     switch (b) {
-      case BIN_G4:
-        LAUNCH(k_sweep_small<4>, grid_for(n * 4, 256, cap), 256, 0, s_, a, lo, hi);
+      default:
+        TRY(launch_short_bin(b, lo, hi, a));
         break;
-      case BIN_G8:
-        LAUNCH(k_sweep_small<8>, grid_for(n * 8, 256, cap), 256, 0, s_, a, lo, hi);
-        break;
-      case BIN_G16:
-        LAUNCH(k_sweep_small<16>, grid_for(n * 16, 256, cap), 256, 0, s_, a, lo, hi);
-        break;
-      case BIN_G32:
-        LAUNCH(k_sweep_small<32>, grid_for(n * 32, 256, cap), 256, 0, s_, a, lo, hi);
-        break;
-      case BIN_WARP: {
-        const size_t smem = 8 * kWarpCap * (sizeof(double) + sizeof(int32_t));
-        LAUNCH(k_sweep_warp<kWarpCap>, grid_for(n * 32, 256, cap), 256, smem, s_, a, lo, hi);
-        break;
-      }
       case BIN_T128:
       case BIN_T256:
       case BIN_BLOCK: {

@@ -1,7 +1,8 @@
 // Ordered accumulation (verify mode on non-integral weights): every
 // per-community sum is folded in CSR order, every community total in vertex
 // order, as the reference's one-thread loop adds them.  A colour class is two
-// launches, the rows of all degree bins and the totals.
+// launches, the rows of all degree bins and the totals; bins of many short rows
+// (kOrdOwnItems) have a launch of their own.
 //
 // What bounds it: latency, launch by launch.  With a launch per degree bin, long
 // rows walked by one warp (a round of 32 entries about 1 us), and a radix sort
@@ -25,6 +26,12 @@ constexpr int kOrdWarps = kOrdThreads / 32;
 constexpr int kOrdChunk = 512;
 constexpr int kOrdTableCap = 8192;      // table_cap(4095): rows up to the block bin
 constexpr int kOrdWarpCap = 256;        // table_cap(127)
+// Rows of a bin for each warp of k_sweep_ordered from which the bin has a launch of
+// its own, with 64 warps per SM instead of 16: a step of all vertices (the basic
+// driver, 1M vertices of 20 entries) 93.8 -> 73.3 ms a run (75.5 with a launch per
+// bin everywhere), 300k 28.6 -> 23.9; limits of 1 to 8 measure the same, 16 takes 3 %
+// more.  Below it the launches cost more than the warps: classes of R-MAT 15.
+constexpr int64_t kOrdOwnItems = 2;
 
 struct OrderedShared {
   int32_t c[kOrdChunk];
