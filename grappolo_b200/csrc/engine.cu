@@ -1262,8 +1262,8 @@ static int upload(cudaStream_t s, T *dst, const std::vector<T> &src) {
   return GLV_OK;
 }
 
-// Hub tables and work lists.  With `tables` (ordered accumulation: one warp
-// walks each hub) every hub gets a table region, reused from step to step;
+// Hub tables and work lists.  With `tables` (ordered accumulation: one
+// block walks each hub) every hub gets a table region, reused from step to step;
 // otherwise every hub's row is cut into chunks and partitions (hub.cuh).
 constexpr size_t kHubStepSlots = size_t(1) << 28;  // hub table slots or pairs of one step (3 GB)
 
