@@ -384,6 +384,10 @@ static int row_entries(cudaStream_t s, int64_t nv, int64_t nk, const int64_t *or
 // edges are repeats: 20M edges over 1000 vertices 1.39 ms by sorting all entries,
 // 1.59 that way, 1.07 this way.)
 constexpr int kDropBlock = 128;  // places to a count
+// Counts that one block makes alone, in one launch for three: with the three
+// 300,000 edges took 237.8 us for 234.5, 20,463 edges 6 % more; a million edges
+// take the same either way.
+constexpr int kDropOneBlock = 4096;
 struct KeptSorted {
   int64_t nge = 0, ndrop = 0;
   uint64_t *key = nullptr;    // kept edges by (head, tail): head << bits | tail
@@ -409,7 +413,10 @@ constexpr int kRunThreads = 256;
 constexpr int kRunTile = kRunThreads * kRunItems;  // runs start in different banks
 
 __global__ void k_pair_keys32(int64_t ne, EdgeView ev, int64_t nv, int bits, uint64_t *keys,
-                              int32_t *idx, int32_t *bad) {
+                              int32_t *idx, int32_t *bad, int64_t words, uint32_t *dropped) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < words;
+       i += (int64_t)gridDim.x * blockDim.x)
+    dropped[i] = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ne;
        i += (int64_t)gridDim.x * blockDim.x) {
     int64_t h = ev.h(i), t = ev.t(i);
@@ -478,20 +485,57 @@ __global__ void __launch_bounds__(256) k_pick(int64_t ne, int bits, const uint64
   }
 }
 
+// The holes among the places of count b (bits w), of which `at` stand before.
+__device__ __forceinline__ void emit_holes(int64_t b, const uint4 &w, int64_t at, int64_t nge,
+                                           int32_t *hole) {
+  const uint32_t part[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    for (uint32_t rem = part[q]; rem; rem &= rem - 1) {
+      const int64_t place = b * kDropBlock + 32 * q + __ffs(rem) - 1;
+      if (place < nge) hole[at++] = (int32_t)place;
+    }
+}
+
 // The holes in order; one thread per kDropBlock places.
 __global__ void k_holes(int64_t nge, const uint4 *words, const int32_t *before, int32_t *hole) {
   const int64_t nb = (nge + kDropBlock - 1) / kDropBlock;
   for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
-       b += (int64_t)gridDim.x * blockDim.x) {
-    const uint4 w = words[b];
-    const uint32_t part[4] = {w.x, w.y, w.z, w.w};
-    int64_t at = before[b];
+       b += (int64_t)gridDim.x * blockDim.x)
+    emit_holes(b, words[b], before[b], nge, hole);
+}
+
+// Counts and holes of a short list (nb <= kDropOneBlock) by one block.
+__global__ void __launch_bounds__(1024) k_drop_index(int nb, int64_t nge, const uint4 *words,
+                                                     int32_t *before, int32_t *hole) {
+  constexpr int kPer = kDropOneBlock / 1024;
+  __shared__ int s_n[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int b0 = threadIdx.x * kPer;
+  uint4 w[kPer];
+  int n = 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      for (uint32_t rem = part[q]; rem; rem &= rem - 1) {
-        const int64_t place = b * kDropBlock + 32 * q + __ffs(rem) - 1;
-        if (place < nge) hole[at++] = (int32_t)place;
-      }
+  for (int k = 0; k < kPer; ++k) {
+    w[k] = b0 + k < nb ? words[b0 + k] : make_uint4(0, 0, 0, 0);
+    n += drop_count(w[k]);
+  }
+  int incl = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_n[warp] = incl;
+  __syncthreads();
+  int at = incl - n;
+  for (int k = 0; k < warp; ++k) at += s_n[k];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    if (b0 + k < nb) {
+      before[b0 + k] = at;
+      emit_holes(b0 + k, w[k], at, nge, hole);
+    }
+    at += drop_count(w[k]);
   }
 }
 
@@ -659,8 +703,10 @@ static int kept_sorted(cudaStream_t s, int64_t nv, int64_t ne, EdgeView ev, DevS
   TRY(d.get(&bad, 1)); TRY(d.get(&cnt, tiles + 1));
   CK(cudaMemsetAsync(bad, 0, sizeof(int32_t), s));
   CK(cudaMemsetAsync(cnt + tiles, 0, sizeof(int64_t), s));
+  const int64_t nb = (ne + kDropBlock - 1) / kDropBlock, nw = nb * (kDropBlock / 32);
+  TRY(d.get(&ks->dropped, nw));
   const int bits = id_bits(nv);
-  k_pair_keys32<<<csr_grid(ne), 256, 0, s>>>(ne, ev, nv, bits, k1, v1, bad);
+  k_pair_keys32<<<csr_grid(ne), 256, 0, s>>>(ne, ev, nv, bits, k1, v1, bad, nw, ks->dropped);
   CK(cudaGetLastError());
   size_t tb = 0, t2 = 0;
   CK(cub::DeviceRadixSort::SortPairs(nullptr, tb, k1, k2, v1, v2, ne, 0, 2 * bits, s));
@@ -679,21 +725,22 @@ static int kept_sorted(cudaStream_t s, int64_t nv, int64_t ne, EdgeView ev, DevS
   ks->key = k1;
   ks->idx = v1;
   ks->ndrop = ne - ks->nge;
-  const int64_t nb = (ne + kDropBlock - 1) / kDropBlock;
-  TRY(d.get(&ks->dropped, nb * (kDropBlock / 32)));
-  CK(cudaMemsetAsync(ks->dropped, 0, nb * (kDropBlock / 8), s));
   k_pick<true><<<(unsigned)tiles, 256, 0, s>>>(ne, bits, k2, v2, cnt, k1, v1, ks->dropped);
   CK(cudaGetLastError());
   *launches += 3;
   if (ks->ndrop > 0 && ks->nge > 0) {
     const uint4 *words = reinterpret_cast<const uint4 *>(ks->dropped);
-    const auto count = thrust::make_transform_iterator(thrust::counting_iterator<int32_t>(0),
-                                                       DropCount{words});
     TRY(d.get(&ks->before, nb)); TRY(d.get(&ks->hole, std::min(ks->nge, ks->ndrop)));
-    CK(cub::DeviceScan::ExclusiveSum(nullptr, t2, count, ks->before, nb, s));
-    TRY(d.get((char **)&temp, (int64_t)t2));
-    CK(cub::DeviceScan::ExclusiveSum(temp, t2, count, ks->before, nb, s));
-    k_holes<<<csr_grid(nb), 256, 0, s>>>(ks->nge, words, ks->before, ks->hole);
+    if (nb <= kDropOneBlock) {
+      k_drop_index<<<1, 1024, 0, s>>>((int)nb, ks->nge, words, ks->before, ks->hole);
+    } else {
+      const auto count = thrust::make_transform_iterator(thrust::counting_iterator<int32_t>(0),
+                                                         DropCount{words});
+      CK(cub::DeviceScan::ExclusiveSum(nullptr, t2, count, ks->before, nb, s));
+      TRY(d.get((char **)&temp, (int64_t)t2));
+      CK(cub::DeviceScan::ExclusiveSum(temp, t2, count, ks->before, nb, s));
+      k_holes<<<csr_grid(nb), 256, 0, s>>>(ks->nge, words, ks->before, ks->hole);
+    }
     ++*launches;
     CK(cudaGetLastError());
   }

@@ -33,3 +33,24 @@ def test_repeats(oracle, n, distinct, order):
                                          torch.tensor(w, device='cuda'), True, True)
     assert np.array_equal(p.cpu().numpy(), ptrs[:nv + 1])
     assert np.array_equal(dt.cpu().numpy(), ot) and np.array_equal(dw.cpu().numpy(), ow)
+
+
+@pytest.mark.parametrize('n', [128 * 1024, 128 * 1024 + 1, 128 * 4096 - 1, 128 * 4096, 128 * 4096 + 1])
+def test_counts_by_one_block_and_by_scan(oracle, n):
+    """Lists on both sides of the limit of the counts that one block makes."""
+    import torch
+    rng = np.random.default_rng(n)
+    nv = n // 16
+    h, t = rng.integers(0, nv, n), rng.integers(0, nv, n)
+    again = rng.integers(0, n, n // 3)
+    put = rng.permutation(n)[:n // 3]
+    h[put], t[put] = t[again], h[again]
+    w = np.arange(1, n + 1) / 8.0
+    rh, rt, rw, nge = oracle.remove_edges(nv, h, t, w)
+    ptrs, sh, st, sw = oracle.sort_edges_undirected(nv, rh[:nge], rt[:nge], rw[:nge])
+    _, ot, ow = oracle.sort_node_edges(nv, ptrs, sh, st, sw)
+    p, dt, dw = louvain.build_csr_device(nv, torch.tensor(h, device='cuda'),
+                                         torch.tensor(t, device='cuda'),
+                                         torch.tensor(w, device='cuda'), True, True)
+    assert np.array_equal(p.cpu().numpy(), ptrs[:nv + 1])
+    assert np.array_equal(dt.cpu().numpy(), ot) and np.array_equal(dw.cpu().numpy(), ow)
